@@ -149,10 +149,10 @@ S2D_API int s2d_integrate_steps(s2d_handle* h, int32_t n, double dt);
  * environment variable S2D_HOST_IO=copy, read by s2d_create, forces the
  * copies for that handle.
  *
- * Every kernel of a step is launched as a programmatic dependent of the one
- * before it on the handle's stream (it waits for its predecessor to complete
- * before touching memory, so results are the same bit for bit);
- * S2D_PDL=0, read by s2d_create, gives plain stream order. */
+ * The kernels of a small FP32 run's step are launched as programmatic
+ * dependents of the one before on the handle's stream (each waits for its
+ * predecessor to complete before touching memory, so results are the same bit
+ * for bit); S2D_PDL=0 or 1, read by s2d_create, sets it for every size. */
 S2D_API int s2d_integrate_one_step_host(s2d_handle* h, double* wC, double* psiC,
                                         int32_t cISize, int32_t nyG, double dt);
 

@@ -24,6 +24,8 @@
 // and keeps the fastest; the state is restored afterwards.
 #include "s2d.h"
 #include "s2d_internal.h"
+#include "s2d_f32step.cuh"
+#include "s2d_fxstep.cuh"
 #include "s2d_step.cuh"
 
 #include <cuda_runtime.h>
@@ -69,7 +71,7 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 // variant that contains it (at 64 registers a 256^2 FP32 stage took 1.11
 // instead of 1.62 ms).
 template <typename T, bool X32>
-__global__ void __launch_bounds__(512) k_batch_stage(const RunDev<T>* __restrict__ runs, int nruns,
+__global__ void __launch_bounds__(512, sizeof(T) == 4 && !X32 ? 2 : 1) k_batch_stage(const RunDev<T>* __restrict__ runs, int nruns,
                                                      const int4* __restrict__ tasks, int ntasks, int stage,
                                                      int* ctrl, int* done, unsigned int* flags) {
     using VT = typename Vec<T>::t;
@@ -115,9 +117,13 @@ __global__ void __launch_bounds__(512) k_batch_stage(const RunDev<T>* __restrict
                 fs.op[1] = OP_V;
                 fs.out[0] = R.I0;
                 fs.out[1] = R.I1;
-                yinv_body<T>(R.d, stage <= 1 ? R.S0 : R.S1, R.rk2, fs, R.tw, R.G12, blk, bufs);
+                const auto* S = stage <= 1 ? R.S0 : R.S1;
+                if (!R.d.direct) yinv_body<T>(R.d, S, R.rk2, fs, R.tw, R.G12, blk, bufs);
+                else if constexpr (sizeof(T) == 8)
+                    fx_yinv_body<12>(R.d, S, R.rk2, fs, (const FxTw*)R.tw, R.G12, blk, bufs);
+                else f32_yinv_body<12>(R.d, S, R.rk2, fs, R.tw, R.G12, blk, bufs);
             } else if (ph == 1) {
-                bool done32 = false;
+                bool done = false;
                 if constexpr (sizeof(T) == 4 && X32) {
                     // FP32 rows of M = 3072: the register radix-12/16 x-pass of
                     // the single run (k_xpass32), one row per 256 threads
@@ -125,13 +131,27 @@ __global__ void __launch_bounds__(512) k_batch_stage(const RunDev<T>* __restrict
                         const int g = threadIdx.x / 256, y = blk * R.G12 + g;
                         xpass32_m3072_row(R.d, R.I0, R.I1, R.tw, y, y < R.d.rows && g < R.G12,
                                           threadIdx.x - g * 256, bufs + (size_t)g * kX32Buf);
-                        done32 = true;
+                        done = true;
                     }
                 }
-                if (!done32) xpass_bas_body<T>(R.d, R.I0, R.I1, R.tw, R.G12, (T)1, blk, bufs);
+                if (done) {
+                } else if (!R.d.direct) {
+                    xpass_bas_body<T>(R.d, R.I0, R.I1, R.tw, R.G12, (T)1, blk, bufs);
+                } else if constexpr (sizeof(T) == 8) {
+                    fx_xpass_body<12>(R.d, R.I0, R.I1, (const FxTw*)R.tw, R.G12, 1.0, blk, bufs);
+                } else {
+                    f32_xpass_body<12>(R.d, R.I0, R.I1, R.tw, R.G12, 1.f, blk, bufs);
+                }
             } else {
-                bad |= yfwd_body<T>(R.d, R.I0, R.I1, R.S0, R.S1, nullptr, R.src, stage, R.dt, R.ph, R.tw, R.G3,
-                                    blk, bufs);
+                if (!R.d.direct)
+                    bad |= yfwd_body<T>(R.d, R.I0, R.I1, R.S0, R.S1, nullptr, R.src, stage, R.dt, R.ph, R.tw, R.G3,
+                                        blk, bufs);
+                else if constexpr (sizeof(T) == 8)
+                    bad |= fx_yfwd_body<12>(R.d, R.I0, R.I1, R.S0, R.S1, nullptr, R.src, stage, R.dt, R.ph,
+                                            (const FxTw*)R.tw, R.G3, blk, bufs);
+                else
+                    bad |= f32_yfwd_body<12>(R.d, R.I0, R.I1, R.S0, R.S1, nullptr, R.src, stage, R.dt, R.ph, R.tw,
+                                             R.G3, blk, bufs);
             }
         }
         __syncthreads();
@@ -351,7 +371,7 @@ S2D_API int s2d_batch_create(int32_t nruns, const s2d_config* cfgs, s2d_batch** 
     cudaDeviceProp prop{};
     if (cudaGetDeviceProperties(&prop, b->device) != cudaSuccess) return bail(berr(S2D_ERR_CUDA, "device query"));
     b->sms = prop.multiProcessorCount;
-    b->max_smem = (int)prop.sharedMemPerBlockOptin - 1024;
+    b->max_smem = (int)prop.sharedMemPerBlockOptin - kStaticSmem;
     for (int i = 0; i < nruns; ++i) {
         s2d_handle* h = nullptr;
         const int r = create_handle(&cfgs[i], b->stream, &h);

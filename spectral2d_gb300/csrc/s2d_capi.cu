@@ -57,12 +57,30 @@ int fail(int code, const char* fmt, ...) {
         if (r_ != S2D_OK) return r_;    \
     } while (0)
 
-// FMA-form twiddle blocks of a plan (s2d_plan.h) in a vector.
+// Per-pass twiddle blocks of a plan (s2d_plan.h) in a vector.
 template <typename T>
-std::vector<TwEnt<T>> fma_tables(Dims* d) {
-    std::vector<TwEnt<T>> tab((size_t)fma_table_entries(*d));
-    fill_fma_tables<T>(d, tab.data(), (int)tab.size());
+std::vector<typename TwTab<T>::t> pass_tables(Dims* d) {
+    std::vector<typename TwTab<T>::t> tab((size_t)table_entries<T>(*d));
+    fill_tables<T>(d, tab.data(), (int)tab.size());
     return tab;
+}
+
+// Builds the plan's twiddle blocks, sets its offsets in *d and copies them to
+// the handle's table (s2d_create and s2d_set_fft_plan).
+int upload_tables(s2d_handle* h, Dims* d) {
+    auto put = [&](size_t at, const void* src, size_t bytes) {
+        return bytes == 0 || cudaMemcpy((char*)h->tw + at, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    };
+    if (h->prec == S2D_FP64) {
+        const auto t = pass_tables<double>(d);
+        if (t.size() * sizeof(t[0]) > h->tab_cap) return fail(S2D_ERR_UNSUPPORTED, "twiddle table too big");
+        if (!put(d->tab_bytes, t.data(), t.size() * sizeof(t[0]))) return fail(S2D_ERR_CUDA, "twiddle upload failed");
+        return S2D_OK;
+    }
+    const auto t = pass_tables<float>(d);
+    if (t.size() * sizeof(t[0]) > h->tab_cap) return fail(S2D_ERR_UNSUPPORTED, "twiddle table too big");
+    if (!put(d->tab_bytes, t.data(), t.size() * sizeof(t[0]))) return fail(S2D_ERR_CUDA, "twiddle upload failed");
+    return S2D_OK;
 }
 
 int kIntMaxBins(int kxMG, int kyMG) {
@@ -114,8 +132,10 @@ cudaError_t round_to_f32(const double* in, float* out, long n, cudaStream_t st) 
 // stream's work
 template <typename T>
 int launch_rhs_stage(s2d_handle* h, int stage, double dt, cudaEvent_t* ev, cudaEvent_t join = nullptr) {
-    const Dims& d = h->d;
     const bool bas = h->ph.form == S2D_NL_BASDEVANT;
+    const bool small = h->small && h->d.direct;   // (other radix plans take the general kernels)
+    Dims d = h->d;
+    if (small) d.Tg = d.M / 4;
     FieldSet fs{};
     fs.nf = bas ? 2 : 3;
     // Basdevant: the scaled factors of u and v from their tables
@@ -131,12 +151,12 @@ int launch_rhs_stage(s2d_handle* h, int stage, double dt, cudaEvent_t* ev, cudaE
     fs.out[2] = h->I[2];
     const void* win = (stage <= 1) ? h->S0 : h->S1;
     if (ev) S2D_CUDA(cudaEventRecord(ev[0], h->stream));
-    S2D_CUDA(Kern<T>::yinv(d, win, bas ? h->rk2s : h->rk2, fs, h->tw, h->stream, h->L_yinv));
+    S2D_CUDA(Kern<T>::yinv(d, win, bas ? h->rk2s : h->rk2, fs, h->tw, h->stream, small ? h->S_yinv : h->L_yinv));
     if (ev) S2D_CUDA(cudaEventRecord(ev[1], h->stream));
-    if (bas) S2D_CUDA(Kern<T>::xpass_bas(d, h->I[0], h->I[1], h->tw, h->stream, h->L_xrow, true));
-    else S2D_CUDA(Kern<T>::xpass_rhs(d, h->I[0], h->I[1], h->I[2], h->tw, h->stream, h->L_xpass));
+    if (bas) S2D_CUDA(Kern<T>::xpass_bas(d, h->I[0], h->I[1], h->tw, h->stream, small ? h->S_xrow : h->L_xrow, true));
+    else S2D_CUDA(Kern<T>::xpass_rhs(h->d, h->I[0], h->I[1], h->I[2], h->tw, h->stream, h->L_xpass));
     if (ev) S2D_CUDA(cudaEventRecord(ev[2], h->stream));
-    if (h->Fv) {
+    if (h->Fv && !small) {
         // K3 in two launches (FP64, Basdevant): the column FFTs take three
         // CTAs per SM; the products' spectra go through I[2] (free in this
         // form) and Fv in the compact layout
@@ -146,7 +166,7 @@ int launch_rhs_stage(s2d_handle* h, int stage, double dt, cudaEvent_t* ev, cudaE
         S2D_CUDA(Kern<T>::stage(d, h->I[2], h->Fv, h->S0, h->S1, h->Sdw, h->src, stage, dt, h->ph, h->flags,
                                 h->stream, h->L_ycol.pdl && !join, h->cc, h->vk));
     } else {
-        Launch L = h->L_yfwd;
+        Launch L = small ? h->S_yfwd : h->L_yfwd;
         if (join) {
             S2D_CUDA(cudaStreamWaitEvent(h->stream, join, 0));
             L.pdl = false;
@@ -487,7 +507,7 @@ int s2d::create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handl
     cudaDeviceProp prop{};
     if (cudaGetDeviceProperties(&prop, h->device) != cudaSuccess)
         return bail(fail(S2D_ERR_CUDA, "cudaGetDeviceProperties failed"));
-    h->max_smem = (int)prop.sharedMemPerBlockOptin - 1024;
+    h->max_smem = (int)prop.sharedMemPerBlockOptin - kStaticSmem;
     h->sms = prop.multiProcessorCount;
     {
         const char* io = std::getenv("S2D_HOST_IO");
@@ -541,22 +561,18 @@ int s2d::create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handl
             S2D_ALLOC(h->fv32, (size_t)d.KX * d.ldS * sizeof(float));
         }
     }
-    // complex twiddles (M entries) followed by the FMA-form blocks
-    std::vector<TwEnt<double>> tabd;
-    std::vector<TwEnt<float>> tabf;
-    if (h->prec == S2D_FP64) tabd = fma_tables<double>(&d);
-    else tabf = fma_tables<float>(&d);
-    d.tab_bytes = (long long)(((size_t)d.M * h->vsz + 63) / 64 * 64);
-    const size_t tab_size = h->prec == S2D_FP64 ? tabd.size() * sizeof(TwEnt<double>)
-                                                : tabf.size() * sizeof(TwEnt<float>);
+    // FP32: complex twiddles (M entries) followed by the per-pass blocks;
+    // FP64: the blocks alone
+    d.tab_bytes = h->prec == S2D_FP64 ? 0 : (long long)(((size_t)d.M * h->vsz + 63) / 64 * 64);
     {
-        // room for the FMA-form blocks of every radix plan (s2d_set_fft_plan)
-        size_t cap = tab_size;
+        // room for the blocks of every radix plan (s2d_set_fft_plan)
+        size_t cap = 0;
         for (int p = 0; p < kNumPlans; ++p) {
             Dims dp = d;
             if (factor_plan(d.M, &dp, p))
-                cap = std::max(cap, (size_t)fma_table_entries(dp) *
-                                        (h->prec == S2D_FP64 ? sizeof(TwEnt<double>) : sizeof(TwEnt<float>)));
+                cap = std::max(cap, h->prec == S2D_FP64
+                                        ? (size_t)table_entries<double>(dp) * sizeof(TwTab<double>::t)
+                                        : (size_t)table_entries<float>(dp) * sizeof(TwTab<float>::t));
         }
         h->tab_cap = cap;
     }
@@ -570,19 +586,14 @@ int s2d::create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handl
 
     // twiddles exp(-2 pi i t / M)
     {
-        std::vector<double> twd(2 * (size_t)d.M);
-        fill_twiddles(d.M, twd.data());
-        if (h->prec == S2D_FP64) {
-            if (cudaMemcpy(h->tw, twd.data(), twd.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
-                return bail(fail(S2D_ERR_CUDA, "twiddle upload failed"));
-        } else {
+        if (h->prec == S2D_FP32) {
+            std::vector<double> twd(2 * (size_t)d.M);
+            fill_twiddles(d.M, twd.data());
             std::vector<float> twf(twd.begin(), twd.end());
             if (cudaMemcpy(h->tw, twf.data(), twf.size() * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
                 return bail(fail(S2D_ERR_CUDA, "twiddle upload failed"));
         }
-        const void* src = h->prec == S2D_FP64 ? (const void*)tabd.data() : (const void*)tabf.data();
-        if (tab_size && cudaMemcpy((char*)h->tw + d.tab_bytes, src, tab_size, cudaMemcpyHostToDevice) != cudaSuccess)
-            return bail(fail(S2D_ERR_CUDA, "twiddle table upload failed"));
+        if (upload_tables(h, &d) != S2D_OK) return bail(S2D_ERR_CUDA);
     }
     if (Kern<double>::init_rk2(d, h->rk2, h->stream) != cudaSuccess ||
         (h->rk2s && Kern<double>::init_rk2(d, h->rk2s, h->stream, std::sqrt(0.5) / (double)d.M) != cudaSuccess) ||
@@ -601,25 +612,50 @@ int s2d::create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handl
     if ((rr = pick_launch(h, d.Tg, tb, tgt, (long)nf * d.KX, &h->L_yinv, "inverse y-pass")) != S2D_OK)
         return bail(rr);
     if ((rr = pick_launch(h, d.Tg, 2 * tb, tgt, d.M / 2, &h->L_xpass, "x-pass")) != S2D_OK) return bail(rr);
-    {
-        // forward y-pass: G columns x 2 fields, run in rounds of c transforms
+    // forward y-pass: G columns x 2 fields, run in rounds of c transforms
+    auto pick_yfwd = [&](int Tg, Launch* out_l) {
         Launch L{};
-        if ((rr = pick_launch(h, d.Tg, 2 * tb, tgt, d.KX, &L, "forward y-pass")) != S2D_OK) return bail(rr);
-        int c = std::max(1, std::min(2 * L.G, tgt / d.Tg));
+        const int e = pick_launch(h, Tg, 2 * tb, tgt, d.KX, &L, "forward y-pass");
+        if (e != S2D_OK) return e;
+        int c = std::max(1, std::min(2 * L.G, tgt / Tg));
         while ((2 * L.G) % c) --c;
-        L.threads = c * d.Tg;
-        h->L_yfwd = L;
+        L.threads = c * Tg;
+        *out_l = L;
+        return (int)S2D_OK;
+    };
+    if ((rr = pick_yfwd(d.Tg, &h->L_yfwd)) != S2D_OK) return bail(rr);
+    // Small grids take 4 elements per thread: with 12 they have under ten warps
+    // per SM and each kernel's time is one transform's latency.  us per step
+    // with 4 / 12 elements:
+    //   FP64  256^2 78 / 139, 384^2 124 / 158, 512^2 160 / 186, 576^2 231 / 244,
+    //         648^2 342 / 344, 768^2 479 / 355
+    //   FP32  256^2 45 / 59, 512^2 73 / 78, 768^2 142 / 156, 864^2 220 / 235,
+    //         1024^2 225 / 223
+    h->small = d.M <= (h->prec == S2D_FP64 ? 864 : 1296);
+    if (h->small) {
+        const int Ts = d.M / 4;
+        if ((rr = pick_launch(h, Ts, tb, tgt, (long)nf * d.KX, &h->S_yinv, "inverse y-pass")) != S2D_OK ||
+            (rr = pick_launch(h, Ts, tb, tgt, d.M, &h->S_xrow, "row transform")) != S2D_OK ||
+            (rr = pick_launch(h, Ts, tb, tgt, d.KX, &h->S_ystore, "column transform")) != S2D_OK ||
+            (rr = pick_yfwd(Ts, &h->S_yfwd)) != S2D_OK)
+            return bail(rr);
     }
     if ((rr = pick_launch(h, d.Tg, tb, tgt, d.M, &h->L_xrow, "row transform")) != S2D_OK) return bail(rr);
     if ((rr = pick_launch(h, d.Tg, tb, tgt, d.KX, &h->L_ystore, "column transform")) != S2D_OK) return bail(rr);
     if ((rr = pick_launch(h, d.Tg, tb, tgt, 2L * d.KX, &h->L_ycol, "forward y-pass (split)")) != S2D_OK)
         return bail(rr);
-    // every kernel of a step is launched as a programmatic dependent of the
-    // one before it (S2D_PDL=0: plain stream order)
+    // The kernels of a small FP32 run's step are launched as programmatic
+    // dependents of the one before (us per step with / without: 64^2 33 / 36,
+    // 128^2 34 / 37, 256^2 43 / 46).  Larger grids and FP64 are not: CTAs that
+    // are resident early fill the SMs that have room and leave the others
+    // short (FP32 288^2 55 / 51, 432^2 107 / 85; FP64 96^2 72 / 66, 256^2 82 /
+    // 78, 768^2 387 / 353).  S2D_PDL=0 / 1 sets it for every size.
     {
         const char* e = std::getenv("S2D_PDL");
-        const bool pdl = !(e && e[0] == '0');
-        for (Launch* L : {&h->L_yinv, &h->L_xpass, &h->L_yfwd, &h->L_xrow, &h->L_ystore, &h->L_ycol}) L->pdl = pdl;
+        const bool pdl = e ? e[0] != '0' : h->prec == S2D_FP32 && d.M <= 384;
+        for (Launch* L : {&h->L_yinv, &h->L_xpass, &h->L_yfwd, &h->L_xrow, &h->L_ystore, &h->L_ycol, &h->S_yinv, &h->S_xrow, &h->S_yfwd,
+                          &h->S_ystore})
+            L->pdl = pdl;
     }
 
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return bail(fail(S2D_ERR_CUDA, "setup failed"));
@@ -669,19 +705,7 @@ S2D_API int s2d_set_fft_plan(s2d_handle* h, int32_t plan) {
     Dims d = h->d;
     if (!factor_plan(d.M, &d, plan)) return fail(S2D_ERR_UNSUPPORTED, "radix plan %d does not apply", plan);
     S2D_CUDA(cudaStreamSynchronize(h->stream));
-    if (h->prec == S2D_FP64) {
-        const std::vector<TwEnt<double>> t = fma_tables<double>(&d);
-        if (t.size() * sizeof(TwEnt<double>) > h->tab_cap) return fail(S2D_ERR_UNSUPPORTED, "twiddle table too big");
-        if (!t.empty())
-            S2D_CUDA(cudaMemcpy((char*)h->tw + d.tab_bytes, t.data(), t.size() * sizeof(TwEnt<double>),
-                                cudaMemcpyHostToDevice));
-    } else {
-        const std::vector<TwEnt<float>> t = fma_tables<float>(&d);
-        if (t.size() * sizeof(TwEnt<float>) > h->tab_cap) return fail(S2D_ERR_UNSUPPORTED, "twiddle table too big");
-        if (!t.empty())
-            S2D_CUDA(cudaMemcpy((char*)h->tw + d.tab_bytes, t.data(), t.size() * sizeof(TwEnt<float>),
-                                cudaMemcpyHostToDevice));
-    }
+    S2D_TRY(upload_tables(h, &d));
     h->d = d;
     h->plan = plan;
     drop_graph(h);   // the step's graph holds the old plan's Dims
@@ -1033,7 +1057,7 @@ S2D_API int s2d_time_steps(s2d_handle* h, int32_t n, double dt, double* ms, doub
 
 S2D_API int s2d_kernels_per_step(const s2d_handle* h) {
     if (!h) return fail(S2D_ERR_INVALID, "null handle");
-    return h->Fv ? 12 : 9;
+    return h->Fv && !(h->small && h->d.direct) ? 12 : 9;
 }
 
 S2D_API int s2d_host_alloc(size_t bytes, void** ptr) {

@@ -24,6 +24,7 @@
 // RK3 stages of the step.
 #include "s2d.h"
 #include "s2d_internal.h"
+#include "s2d_f32step.cuh"
 #include "s2d_step.cuh"
 
 #include <cuda.h>
@@ -1456,7 +1457,7 @@ struct LesRun {
     typename Vec<T>::t* I1;
     typename Vec<T>::t* I2;
     typename Vec<T>::t* src;   // -Pi^ (compact layout)
-    double* part;   // sums of |w^|^2 per column tile of k_cl_yinv; part[nparts]: their total
+    double* part;   // sums of |w^|^2 per column (k_cl_yinv); part[KX]: their total
 };
 
 // Sum of the nparts partial sums by one warp in a fixed order (lane l adds
@@ -1470,12 +1471,15 @@ __device__ __forceinline__ double warp_ordered_sum(const double* __restrict__ pa
     return s;
 }
 
+// The closure transforms run E elements per thread; E = 4 (small grids, one
+// run) needs FP32 and a direct plan (s2d_f32step.cuh).
+
 // K1 of (w, psi): inverse y-pass of every run's state.  The CTAs of the w
 // field also sum |w^|^2 over their columns (kx > 0 twice: the other half of
 // the spectrum), which by Parseval is the mean of w^2 over the collocation
-// grid (the inverse transform is unnormalised); per thread, then a fixed
-// tree over the CTA, into part[column tile].
-template <typename T>
+// grid (the inverse transform is unnormalised): one warp per column, lanes
+// over the rows and an xor butterfly, into part[kx], whatever the tile shape.
+template <typename T, int E>
 __global__ void __launch_bounds__(512) k_cl_yinv(Dims d, const LesRun<T>* __restrict__ runs,
                                                   const double* __restrict__ rk2,
                                                   const typename Vec<T>::t* __restrict__ tw, int G) {
@@ -1489,44 +1493,42 @@ __global__ void __launch_bounds__(512) k_cl_yinv(Dims d, const LesRun<T>* __rest
     fs.op[1] = OP_PSI;
     fs.out[0] = R.I0;
     fs.out[1] = R.I1;
-    yinv_body<T>(d, R.S0, rk2, fs, tw, G, blockIdx.x, reinterpret_cast<VT*>(smem_raw));
     const int ncg = (d.KX + G - 1) / G;
-    if ((int)blockIdx.x >= ncg) return;   // the psi field's CTAs (uniform per CTA)
-    const int kx0 = blockIdx.x * G;
-    const int gtot = min(G, d.KX - kx0);
-    const DivBy byKY(d.KY);
-    double s = 0.0;
-    for (int idx = threadIdx.x; idx < gtot * d.KY; idx += blockDim.x) {
-        const int gg = byKY(idx);
-        const int kx = kx0 + gg;
-        const VT v = __ldcg(&R.S0[(size_t)kx * d.ldS + (idx - gg * d.KY)]);
-        const double m = (double)v.x * (double)v.x + (double)v.y * (double)v.y;
-        s += kx > 0 ? 2.0 * m : m;
+    if ((int)blockIdx.x < ncg) {   // the w field's CTAs
+        const int nw = blockDim.x >> 5, lane = threadIdx.x & 31;
+        for (int gg = threadIdx.x >> 5; gg < G; gg += nw) {
+            const int kx = blockIdx.x * G + gg;
+            if ((int)(threadIdx.x >> 5) >= nw || kx >= d.KX) break;   // whole warps only
+            double s = 0.0;
+            for (int jc = lane; jc < d.KY; jc += 32) {
+                const VT v = __ldcg(&R.S0[(size_t)kx * d.ldS + jc]);
+                s += (double)v.x * (double)v.x + (double)v.y * (double)v.y;
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) R.part[kx] = kx > 0 ? 2.0 * s : s;
+        }
     }
-    // tree over the CTA in the (now free) FFT buffers: G*M*vsz >= 8 B per thread
-    double* red = reinterpret_cast<double*>(smem_raw);
-    __syncthreads();
-    red[threadIdx.x] = s;
-    __syncthreads();
-    int w = 1;
-    while (w < (int)blockDim.x) w <<= 1;
-    for (w >>= 1; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w && threadIdx.x + w < blockDim.x) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
+    VT* bufs = reinterpret_cast<VT*>(smem_raw);
+    if constexpr (sizeof(T) == 4) {
+        if (d.direct) {
+            f32_yinv_body<E>(d, R.S0, rk2, fs, tw, G, blockIdx.x, bufs);
+            return;
+        }
     }
-    if (threadIdx.x == 0) R.part[blockIdx.x] = red[0];
+    if constexpr (E == kElemsPerThread) yinv_body<T>(d, R.S0, rk2, fs, tw, G, blockIdx.x, bufs);
 }
 
 // Physical rows of w and psi (one inverse FFT of W + i PSI per row), written
 // as the network input of every run: (w / (a s0), psi / (a s1)) in BF16, a =
-// rms w of the run from the nparts sums of k_cl_yinv (their total, the mean
+// rms w of the run from the nparts column sums of k_cl_yinv (their total, the mean
 // of w^2, is kept in part[nparts] for k_cl_xfwd).  Only channels 0 and 1 of
 // x are written: channels 2..15 of the input buffer are zero from its
 // allocation on, and every writer of it keeps them so.  framed: x holds
 // images with the one-pixel circular frame of the fused forward ([M + 2]^2
 // pixels, pixel (y, n) at (y + 1, n + 1)), the border pixels written into the
 // frame as well.
-template <typename T>
+template <typename T, int E>
 __global__ void __launch_bounds__(512) k_cl_xinv(Dims d, const LesRun<T>* __restrict__ runs,
                                                   const typename Vec<T>::t* __restrict__ tw, int G, int nparts,
                                                   float r0, float r1, __nv_bfloat16* x, int framed) {
@@ -1549,37 +1551,54 @@ __global__ void __launch_bounds__(512) k_cl_xinv(Dims d, const LesRun<T>* __rest
     const bool active = y < d.M;
     const int yy = active ? y : 0;
     VT* Z = bufs + (size_t)g * d.M;
-    build_pair(Z, R.I0 + (size_t)yy * d.ldI, R.I1 + (size_t)yy * d.ldI, d, lane, active);
-    fft_run<true>(Z, d, lane, tw);   // begins with a barrier: s_ia is visible after it
-    const T a0 = (T)((double)r0 * s_ia), a1 = (T)((double)r1 * s_ia);
-    if (active && !framed) {
-        uint32_t* xr = reinterpret_cast<uint32_t*>(x + ((size_t)blockIdx.y * d.M + y) * (size_t)d.M * 16);
-        for (int n = lane; n < d.M; n += d.Tg) {
-            const VT z = Z[n];
-            xr[(size_t)n * 8] = pack_bf16((float)(z.x * a0), (float)(z.y * a1));
+    const VT* I0 = R.I0 + (size_t)yy * d.ldI;
+    const VT* I1 = R.I1 + (size_t)yy * d.ldI;
+    const size_t fw = (size_t)d.M + 2;
+    const int wy = y == 0 ? d.M + 1 : (y == d.M - 1 ? 0 : -1);
+    // pixel (y, n) of the network input, with its copies in the frame
+    auto put = [&](int n, VT z, T a0, T a1) {
+        const uint32_t v = pack_bf16((float)(z.x * a0), (float)(z.y * a1));
+        if (!framed) {
+            reinterpret_cast<uint32_t*>(x + ((size_t)blockIdx.y * d.M + y) * (size_t)d.M * 16)[(size_t)n * 8] = v;
+            return;
         }
-    } else if (active) {
-        const size_t fw = (size_t)d.M + 2;
-        const int wy = y == 0 ? d.M + 1 : (y == d.M - 1 ? 0 : -1);
         uint32_t* xr = reinterpret_cast<uint32_t*>(x + ((size_t)blockIdx.y * fw + y + 1) * fw * 16);
         uint32_t* xw = reinterpret_cast<uint32_t*>(x + ((size_t)blockIdx.y * fw + (wy < 0 ? 0 : wy)) * fw * 16);
-        for (int n = lane; n < d.M; n += d.Tg) {
-            const VT z = Z[n];
-            const uint32_t v = pack_bf16((float)(z.x * a0), (float)(z.y * a1));
-            const int wx = n == 0 ? d.M + 1 : (n == d.M - 1 ? 0 : -1);
-            xr[(size_t)(n + 1) * 8] = v;
-            if (wx >= 0) xr[(size_t)wx * 8] = v;
-            if (wy >= 0) {
-                xw[(size_t)(n + 1) * 8] = v;
-                if (wx >= 0) xw[(size_t)wx * 8] = v;
-            }
+        const int wx = n == 0 ? d.M + 1 : (n == d.M - 1 ? 0 : -1);
+        xr[(size_t)(n + 1) * 8] = v;
+        if (wx >= 0) xr[(size_t)wx * 8] = v;
+        if (wy >= 0) {
+            xw[(size_t)(n + 1) * 8] = v;
+            if (wx >= 0) xw[(size_t)wx * 8] = v;
         }
+    };
+    // (the transforms synchronise the CTA: s_ia is visible after them)
+    if constexpr (sizeof(T) == 4) {
+        if (d.direct) {
+            float2 z[kFxNB<E, 4>][4];
+            f32_row_inverse<E>(d, I0, I1, active, tw, lane, Z, z);
+            const T a0 = (T)((double)r0 * s_ia), a1 = (T)((double)r1 * s_ia);
+            if (active) {
+#pragma unroll
+                for (int b = 0; b < kFxNB<E, 4>; ++b)
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) put(lane + b * d.Tg + r * (d.M / 4), z[b][r], a0, a1);
+            }
+            return;
+        }
+    }
+    if constexpr (E == kElemsPerThread) {
+        build_pair(Z, I0, I1, d, lane, active);
+        fft_run<true>(Z, d, lane, tw);
+        const T a0 = (T)((double)r0 * s_ia), a1 = (T)((double)r1 * s_ia);
+        if (active)
+            for (int n = lane; n < d.M; n += d.Tg) put(n, Z[n], a0, a1);
     }
 }
 
 // Network output -> -Pi on the grid (scale a^2 y, scale = -s2), forward x-FFT
 // of row pairs into the half-spectral rows I2.
-template <typename T>
+template <typename T, int E>
 __global__ void __launch_bounds__(512) k_cl_xfwd(Dims d, const LesRun<T>* __restrict__ runs, int nparts,
                                                   const float* __restrict__ Y, double scale,
                                                   const typename Vec<T>::t* __restrict__ tw, int G, T xscale) {
@@ -1598,15 +1617,37 @@ __global__ void __launch_bounds__(512) k_cl_xfwd(Dims d, const LesRun<T>* __rest
     VT* Z = bufs + (size_t)g * d.M;
     const float* r1 = Y + (size_t)blockIdx.y * HW + (size_t)y1 * d.M;
     const float* r2 = r1 + d.M;
-    for (int n = lane; n < d.M; n += d.Tg)
-        Z[n] = active ? mk<VT>(s * (T)r1[n], s * (T)r2[n]) : mk<VT>((T)0, (T)0);
-    fft_run<false>(Z, d, lane, tw);
-    extract_pair(Z, R.I2 + (size_t)y1 * d.ldI, R.I2 + (size_t)(y1 + 1) * d.ldI, d, lane, active, xscale);
+    VT* o1 = R.I2 + (size_t)y1 * d.ldI;
+    VT* o2 = o1 + d.ldI;
+    if constexpr (sizeof(T) == 4) {
+        if (d.direct) {
+            float2 z[kFxNB<E, 4>][4];
+#pragma unroll
+            for (int b = 0; b < kFxNB<E, 4>; ++b)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int n = lane + b * d.Tg + r * (d.M / 4);
+                    z[b][r] = active ? make_float2(s * __ldcg(&r1[n]), s * __ldcg(&r2[n])) : make_float2(0.f, 0.f);
+                }
+            f32_row_forward<E>(d, z, tw, lane, Z, [&](int k, float2 a, float2 c) {
+                if (!active) return;
+                o1[k] = make_float2((a.x + c.x) * xscale, (a.y - c.y) * xscale);
+                o2[k] = make_float2((a.y + c.y) * xscale, (c.x - a.x) * xscale);
+            });
+            return;
+        }
+    }
+    if constexpr (E == kElemsPerThread) {
+        for (int n = lane; n < d.M; n += d.Tg)
+            Z[n] = active ? mk<VT>(s * (T)r1[n], s * (T)r2[n]) : mk<VT>((T)0, (T)0);
+        fft_run<false>(Z, d, lane, tw);
+        extract_pair(Z, o1, o2, d, lane, active, xscale);
+    }
 }
 
 // Forward y-FFT of the columns of I2 with Truncate into src; modes with
 // |k|^2 < kmin2 (the closure's band) are zero.
-template <typename T>
+template <typename T, int E>
 __global__ void __launch_bounds__(512) k_cl_ystore(Dims d, const LesRun<T>* __restrict__ runs,
                                                     const typename Vec<T>::t* __restrict__ tw, int G,
                                                     double kmin2) {
@@ -1619,24 +1660,37 @@ __global__ void __launch_bounds__(512) k_cl_ystore(Dims d, const LesRun<T>* __re
     const int lane = threadIdx.x - g * d.Tg;
     const int kx0 = blockIdx.x * G;
     const int gtot = min(G, d.KX - kx0);
-    const DivBy byG(G), byKY(d.KY);
-    for (int idx = threadIdx.x; idx < G * d.M; idx += blockDim.x) {
-        const int y = byG(idx);
-        const int gg = idx - y * G;
-        bufs[(size_t)gg * d.M + y] = gg < gtot ? __ldcg(&R.I2[(size_t)y * d.ldI + kx0 + gg]) : mk<VT>((T)0, (T)0);
-    }
-    fft_run<false>(bufs + (size_t)g * d.M, d, lane, tw);
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < gtot * d.KY; idx += blockDim.x) {
-        const int gg = byKY(idx);
-        const int jc = idx - gg * d.KY;
-        const int kx = kx0 + gg;
+    auto store = [&](int kx, int jc, VT v) {
         const int ky = ky_of_jc(d, jc);
-        const int n = jc <= d.K ? jc : ky + d.M;
-        VT v = bufs[(size_t)gg * d.M + n];
         const int k2 = kx * kx + ky * ky;
         if (k2 > d.K * d.K || (double)k2 < kmin2) v = mk<VT>((T)0, (T)0);
         R.src[(size_t)kx * d.ldS + jc] = v;
+    };
+    if constexpr (sizeof(T) == 4) {
+        if (d.direct) {
+            f32_yfwd_column<E, false>(d, R.I2, g < gtot, kx0 + g, tw, lane, bufs + (size_t)g * d.M,
+                                      [&](int jc, float2 v) {
+                                          if (g < gtot) store(kx0 + g, jc, v);
+                                      });
+            return;
+        }
+    }
+    if constexpr (E == kElemsPerThread) {
+        const DivBy byG(G), byKY(d.KY);
+        for (int idx = threadIdx.x; idx < G * d.M; idx += blockDim.x) {
+            const int y = byG(idx);
+            const int gg = idx - y * G;
+            bufs[(size_t)gg * d.M + y] =
+                gg < gtot ? __ldcg(&R.I2[(size_t)y * d.ldI + kx0 + gg]) : mk<VT>((T)0, (T)0);
+        }
+        fft_run<false>(bufs + (size_t)g * d.M, d, lane, tw);
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < gtot * d.KY; idx += blockDim.x) {
+            const int gg = byKY(idx);
+            const int jc = idx - gg * d.KY;
+            const int n = jc <= d.K ? jc : ky_of_jc(d, jc) + d.M;
+            store(kx0 + gg, jc, bufs[(size_t)gg * d.M + n]);
+        }
     }
 }
 
@@ -1978,10 +2032,12 @@ int ensure_les_buffers(s2d_handle* h) {
     if (h->device >= 0 && h->device < 64 && !attr[h->device]) {
         C_CUDA(cudaFuncSetAttribute(k_xinv_phys2<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, h->max_smem));
         C_CUDA(cudaFuncSetAttribute(k_xinv_phys2<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, h->max_smem));
-        const void* fns[] = {(const void*)k_cl_yinv<double>, (const void*)k_cl_yinv<float>,
-                             (const void*)k_cl_xinv<double>, (const void*)k_cl_xinv<float>,
-                             (const void*)k_cl_xfwd<double>, (const void*)k_cl_xfwd<float>,
-                             (const void*)k_cl_ystore<double>, (const void*)k_cl_ystore<float>};
+        const void* fns[] = {(const void*)k_cl_yinv<double, 12>, (const void*)k_cl_xinv<double, 12>,
+                             (const void*)k_cl_xfwd<double, 12>, (const void*)k_cl_ystore<double, 12>,
+                             (const void*)k_cl_yinv<float, 12>, (const void*)k_cl_xinv<float, 12>,
+                             (const void*)k_cl_xfwd<float, 12>, (const void*)k_cl_ystore<float, 12>,
+                             (const void*)k_cl_yinv<float, 4>, (const void*)k_cl_xinv<float, 4>,
+                             (const void*)k_cl_xfwd<float, 4>, (const void*)k_cl_ystore<float, 4>};
         for (const void* f : fns)
             C_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, h->max_smem));
         attr[h->device] = true;
@@ -1993,8 +2049,8 @@ int ensure_les_buffers(s2d_handle* h) {
     return S2D_OK;
 }
 
-// LesRun table of n runs followed by M + 1 doubles per run: the partial
-// sums of k_cl_yinv (one per column tile, at most M) and their total.
+// LesRun table of n runs followed by M + 1 doubles per run: the column sums
+// of k_cl_yinv (KX of them) and their total.
 int closure_table_impl(s2d_handle* const* runs, int n, void** tab) {
     const s2d_handle* h0 = runs[0];
     const size_t pstride = (size_t)h0->d.M + 1;
@@ -2025,21 +2081,19 @@ int closure_table_impl(s2d_handle* const* runs, int n, void** tab) {
     return S2D_OK;
 }
 
-template <typename T>
-int closure_terms_t(s2d_cnn* c, s2d_handle* const* runs, int n, const void* tab, cudaStream_t st) {
+template <typename T, int E>
+int closure_terms_e(s2d_cnn* c, s2d_handle* const* runs, int n, const void* tab, cudaStream_t st, const Dims& d,
+                    const Launch& Ly, const Launch& Lx, const Launch& Ls) {
     using VT = typename Vec<T>::t;
     const s2d_handle* h0 = runs[0];
-    const Dims& d = h0->d;
     const LesRun<T>* R = (const LesRun<T>*)tab;
-    const Launch& Ly = h0->L_yinv;
-    const Launch& Lx = h0->L_xrow;
-    const Launch& Ls = h0->L_ystore;
-    const int nparts = (d.KX + Ly.G - 1) / Ly.G;   // k_cl_yinv's column tiles of the w field
+    const int nparts = d.KX;   // k_cl_yinv's column sums
     const VT* tw = (const VT*)h0->tw;
-    const bool pdl = Ly.pdl;
-    C_CUDA(launch_k(k_cl_yinv<T>, dim3(2 * nparts, n), Ly.threads, Ly.smem, st, pdl, d, R, h0->rk2, tw, Ly.G));
+    const bool pdl = Ly.pdl && n == 1;   // (see s2d_create: only grids that leave SMs idle gain)
+    C_CUDA(launch_k(k_cl_yinv<T, E>, dim3(2 * ((d.KX + Ly.G - 1) / Ly.G), n), Ly.threads, Ly.smem, st, pdl, d, R,
+                    h0->rk2, tw, Ly.G));
     const bool fused = c->fused;
-    C_CUDA(launch_k(k_cl_xinv<T>, dim3((d.M + Lx.G - 1) / Lx.G, n), Lx.threads, Lx.smem, st, pdl, d, R, tw, Lx.G,
+    C_CUDA(launch_k(k_cl_xinv<T, E>, dim3((d.M + Lx.G - 1) / Lx.G, n), Lx.threads, Lx.smem, st, pdl, d, R, tw, Lx.G,
                     nparts, (float)(1.0 / c->scale[0]), (float)(1.0 / c->scale[1]), fused ? c->X0f : c->X0,
                     (int)fused));
     // the network runs on the caller's stream: borrow it for the forward pass
@@ -2048,11 +2102,23 @@ int closure_terms_t(s2d_cnn* c, s2d_handle* const* runs, int n, const void* tab,
     const int r = fused ? forward_fused(c, n, true) : forward(c, n, false, pdl);
     c->stream = saved;
     if (r != S2D_OK) return r;
-    C_CUDA(launch_k(k_cl_xfwd<T>, dim3((d.M / 2 + Lx.G - 1) / Lx.G, n), Lx.threads, Lx.smem, st, pdl, d, R,
+    C_CUDA(launch_k(k_cl_xfwd<T, E>, dim3((d.M / 2 + Lx.G - 1) / Lx.G, n), Lx.threads, Lx.smem, st, pdl, d, R,
                     nparts, (const float*)c->Y, -c->scale[2], tw, Lx.G, (T)(0.5 / ((double)d.M * (double)d.M))));
-    C_CUDA(launch_k(k_cl_ystore<T>, dim3((d.KX + Ls.G - 1) / Ls.G, n), Ls.threads, Ls.smem, st, pdl, d, R, tw,
+    C_CUDA(launch_k(k_cl_ystore<T, E>, dim3((d.KX + Ls.G - 1) / Ls.G, n), Ls.threads, Ls.smem, st, pdl, d, R, tw,
                     Ls.G, c->k_min * c->k_min));
     return S2D_OK;
+}
+
+template <typename T>
+int closure_terms_t(s2d_cnn* c, s2d_handle* const* runs, int n, const void* tab, cudaStream_t st) {
+    const s2d_handle* h0 = runs[0];
+    if constexpr (sizeof(T) == 4)
+        if (n == 1 && h0->small && h0->d.direct) {   // latency: 4 elements per thread, as the step
+            Dims d = h0->d;
+            d.Tg = d.M / 4;
+            return closure_terms_e<T, 4>(c, runs, n, tab, st, d, h0->S_yinv, h0->S_xrow, h0->S_ystore);
+        }
+    return closure_terms_e<T, 12>(c, runs, n, tab, st, h0->d, h0->L_yinv, h0->L_xrow, h0->L_ystore);
 }
 
 template <typename T>

@@ -10,13 +10,13 @@
 // 12 of its elements into registers, the CTA synchronises, then every thread
 // writes its results.
 //
-// FP64 on GB300 has a small fraction of the FP32 issue rate, so the code is
-// written to minimise FP64 instructions: twiddles come from a table (a load,
-// not a sincos), twiddled radix-4/2 passes use the FMA form (TwEnt), and the
-// radix-3 and radix-4 butterflies use only additions and FMAs.
+// FP64 values are transformed in 64-bit block fixed point on the integer
+// pipes (fx_run below; the arithmetic is in s2d_fixed.cuh): the first pass
+// converts, the last converts back, the passes in between work on integers.
 //
-// FP32 runs the same passes; with 64x the FP64 rate, its cost is the
-// shared-memory traffic and the barriers of the in-place passes.
+// FP32 runs the passes on floats: twiddles come from a table (a load, not a
+// sincos), twiddled radix-4/2 passes use the FMA form (TwEnt).  Its cost is
+// the shared-memory traffic and the barriers of the in-place passes.
 #pragma once
 
 #include "s2d_internal.h"
@@ -148,16 +148,27 @@ struct DivBy {
     __device__ __forceinline__ int operator()(int n) const { return d == 1 ? n : (int)__umulhi((unsigned)n, m); }
 };
 
+// Butterflies of radix R per thread with E elements per thread (T = M / E
+// threads), and whether butterfly j exists (the last round may be partial
+// when R does not divide E).
+template <int E, int R>
+constexpr int kFxNB = (E + R - 1) / R;
+template <int E, int R>
+__device__ __forceinline__ bool fx_on(int j, int M) {
+    return E % R == 0 || j < M / R;
+}
+
 // One in-place Stockham pass of radix R over the transform in buf.
-template <int R, bool INV, typename VT>
+template <int E, int R, bool INV, typename VT>
 __device__ __forceinline__ void fft_pass(VT* buf, int M, int Ns, unsigned mg, int tstep, int lane, int Tg,
                                          const VT* __restrict__ tw) {
-    constexpr int NB = kElemsPerThread / R;
+    constexpr int NB = kFxNB<E, R>;
     VT v[NB][R];
     const int stride = M / R;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
+        if (!fx_on<E, R>(j, M)) continue;
 #pragma unroll
         for (int r = 0; r < R; ++r) v[b][r] = buf[j + r * stride];
     }
@@ -166,6 +177,7 @@ __device__ __forceinline__ void fft_pass(VT* buf, int M, int Ns, unsigned mg, in
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
+        if (!fx_on<E, R>(j, M)) continue;
         const int k = mod(j);
         if (Ns > 1) {
             const int ts = k * tstep;
@@ -208,14 +220,15 @@ __device__ __forceinline__ void bf3_bzero(VT* v) {
 // truncated to |k| <= K = M/3, so index n is non-zero only for n <= K or
 // n >= M - K.  Butterfly j reads (x[j], x[j + M/3], x[j + 2M/3]); its middle
 // input is zero for j > 0.
-template <bool INV, typename VT>
+template <int E, bool INV, typename VT>
 __device__ __forceinline__ void fft_pass3_midzero(VT* buf, int M, int lane, int Tg) {
-    constexpr int NB = kElemsPerThread / 3;
+    constexpr int NB = kFxNB<E, 3>;
     VT v[NB][3];
     const int stride = M / 3;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
+        if (!fx_on<E, 3>(j, M)) continue;
         v[b][0] = buf[j];
         v[b][1] = buf[j + stride];
         v[b][2] = buf[j + 2 * stride];
@@ -224,6 +237,7 @@ __device__ __forceinline__ void fft_pass3_midzero(VT* buf, int M, int lane, int 
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
+        if (!fx_on<E, 3>(j, M)) continue;
         if (j == 0) bf3<INV>(v[b]);
         else bf3_bzero<INV>(v[b]);
         buf[j * 3] = v[b][0];
@@ -233,12 +247,8 @@ __device__ __forceinline__ void fft_pass3_midzero(VT* buf, int M, int lane, int 
     __syncthreads();
 }
 
-__device__ __forceinline__ double ffma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float ffma(float a, float b, float c) { return fmaf(a, b, c); }
 
-__device__ __forceinline__ double neg_if(double v, int cond) {
-    return __longlong_as_double(__double_as_longlong(v) ^ ((long long)(cond != 0) << 63));
-}
 __device__ __forceinline__ float neg_if(float v, int cond) {
     return __int_as_float(__float_as_int(v) ^ ((cond != 0) << 31));
 }
@@ -265,12 +275,41 @@ __device__ __forceinline__ VT tw_fma(VT x, T t, int q) {
     return r;
 }
 
-// Radix-4 Stockham pass with FMA-form twiddles (Ns > 1): 22 FP64
-// instructions per butterfly instead of 12 (3 complex products) + 16.
-template <bool INV, typename VT, typename T>
+// Radix-4 butterfly with FMA-form twiddles: 22 instructions instead of 12 (3
+// complex products) + 16.
+template <bool INV, typename VT>
+__device__ __forceinline__ void bf4_fma(VT* v, const TwEnt<float>& e) {
+    const VT a = v[0];
+    const VT B = tw_fma<INV>(v[1], e.t1, e.q & 3);
+    const VT Cc = tw_fma<INV>(v[2], e.t2, (e.q >> 2) & 3);
+    const VT D = tw_fma<INV>(v[3], e.t3, (e.q >> 4) & 3);
+    // t0,1 = a +- c2 C ; E,F = B +- (c3/c1) D ; y = t +- c1 E, t -+ i c1 F
+    const float t0x = ffma(e.c2, Cc.x, a.x), t0y = ffma(e.c2, Cc.y, a.y);
+    const float t1x = ffma(-e.c2, Cc.x, a.x), t1y = ffma(-e.c2, Cc.y, a.y);
+    const float Ex = ffma(e.r31, D.x, B.x), Ey = ffma(e.r31, D.y, B.y);
+    const float Fx = ffma(-e.r31, D.x, B.x), Fy = ffma(-e.r31, D.y, B.y);
+    v[0].x = ffma(e.c1, Ex, t0x);
+    v[0].y = ffma(e.c1, Ey, t0y);
+    v[2].x = ffma(-e.c1, Ex, t0x);
+    v[2].y = ffma(-e.c1, Ey, t0y);
+    if (!INV) {  // y1 = t1 - i c1 F, y3 = t1 + i c1 F
+        v[1].x = ffma(e.c1, Fy, t1x);
+        v[1].y = ffma(-e.c1, Fx, t1y);
+        v[3].x = ffma(-e.c1, Fy, t1x);
+        v[3].y = ffma(e.c1, Fx, t1y);
+    } else {
+        v[1].x = ffma(-e.c1, Fy, t1x);
+        v[1].y = ffma(e.c1, Fx, t1y);
+        v[3].x = ffma(e.c1, Fy, t1x);
+        v[3].y = ffma(-e.c1, Fx, t1y);
+    }
+}
+
+// Radix-4 Stockham pass with FMA-form twiddles (Ns > 1).
+template <int E, bool INV, typename VT>
 __device__ __forceinline__ void fft_pass4_fma(VT* buf, int M, int Ns, unsigned mg, int lane, int Tg,
-                                              const TwEnt<T>* __restrict__ tab) {
-    constexpr int NB = kElemsPerThread / 4;
+                                              const TwEnt<float>* __restrict__ tab) {
+    constexpr int NB = kFxNB<E, 4>;
     VT v[NB][4];
     const int stride = M / 4;
 #pragma unroll
@@ -285,46 +324,20 @@ __device__ __forceinline__ void fft_pass4_fma(VT* buf, int M, int Ns, unsigned m
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
         const int k = mod(j);
-        const TwEnt<T> e = tab[k];
-        const VT a = v[b][0];
-        const VT B = tw_fma<INV>(v[b][1], e.t1, e.q & 3);
-        const VT Cc = tw_fma<INV>(v[b][2], e.t2, (e.q >> 2) & 3);
-        const VT D = tw_fma<INV>(v[b][3], e.t3, (e.q >> 4) & 3);
-        // t0,1 = a +- c2 C ; E,F = B +- (c3/c1) D ; y = t +- c1 E, t -+ i c1 F
-        const T t0x = ffma(e.c2, Cc.x, a.x), t0y = ffma(e.c2, Cc.y, a.y);
-        const T t1x = ffma(-e.c2, Cc.x, a.x), t1y = ffma(-e.c2, Cc.y, a.y);
-        const T Ex = ffma(e.r31, D.x, B.x), Ey = ffma(e.r31, D.y, B.y);
-        const T Fx = ffma(-e.r31, D.x, B.x), Fy = ffma(-e.r31, D.y, B.y);
-        VT y0, y1, y2, y3;
-        y0.x = ffma(e.c1, Ex, t0x);
-        y0.y = ffma(e.c1, Ey, t0y);
-        y2.x = ffma(-e.c1, Ex, t0x);
-        y2.y = ffma(-e.c1, Ey, t0y);
-        if (!INV) {  // y1 = t1 - i c1 F, y3 = t1 + i c1 F
-            y1.x = ffma(e.c1, Fy, t1x);
-            y1.y = ffma(-e.c1, Fx, t1y);
-            y3.x = ffma(-e.c1, Fy, t1x);
-            y3.y = ffma(e.c1, Fx, t1y);
-        } else {
-            y1.x = ffma(-e.c1, Fy, t1x);
-            y1.y = ffma(e.c1, Fx, t1y);
-            y3.x = ffma(e.c1, Fy, t1x);
-            y3.y = ffma(-e.c1, Fx, t1y);
-        }
+        const TwEnt<float> e = tab[k];
+        bf4_fma<INV>(v[b], e);
         const int base = (j - k) * 4 + k;
-        buf[base] = y0;
-        buf[base + Ns] = y1;
-        buf[base + 2 * Ns] = y2;
-        buf[base + 3 * Ns] = y3;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) buf[base + r * Ns] = v[b][r];
     }
     __syncthreads();
 }
 
 // Radix-2 Stockham pass with an FMA-form twiddle (Ns > 1): y = a +- c1 B.
-template <bool INV, typename VT, typename T>
+template <int E, bool INV, typename VT>
 __device__ __forceinline__ void fft_pass2_fma(VT* buf, int M, int Ns, unsigned mg, int lane, int Tg,
-                                              const TwEnt<T>* __restrict__ tab) {
-    constexpr int NB = kElemsPerThread / 2;
+                                              const TwEnt<float>* __restrict__ tab) {
+    constexpr int NB = kFxNB<E, 2>;
     VT v[NB][2];
     const int stride = M / 2;
 #pragma unroll
@@ -339,7 +352,7 @@ __device__ __forceinline__ void fft_pass2_fma(VT* buf, int M, int Ns, unsigned m
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
         const int k = mod(j);
-        const T t1 = tab[k].t1, c1 = tab[k].c1;
+        const float t1 = tab[k].t1, c1 = tab[k].c1;
         const int q = tab[k].q;
         const VT a = v[b][0];
         const VT B = tw_fma<INV>(v[b][1], t1, q & 3);
@@ -355,34 +368,278 @@ __device__ __forceinline__ void fft_pass2_fma(VT* buf, int M, int Ns, unsigned m
     __syncthreads();
 }
 
-// Full transform: unnormalised, sign -1 (forward) or +1 (INV).  Every thread
-// of the CTA must call it (it synchronises the CTA); starts with a barrier so
-// that callers may fill buf just before.  tw points at the complex table
-// (M entries) followed, d.tab_bytes later, by the TwEnt table.  Inverse
-// transforms of truncated spectra (input zero for K < n < M - K, K = M/3: the
-// inverse transforms of this library) take the pruned first radix-3 pass.
-template <bool INV, typename VT>
-__device__ __forceinline__ void fft_run(VT* buf, const Dims& d, int lane, const VT* __restrict__ tw) {
-    using T = decltype(buf[0].x);
-    const TwEnt<T>* tab = reinterpret_cast<const TwEnt<T>*>(reinterpret_cast<const char*>(tw) + d.tab_bytes);
+// ---- FP64 in block fixed point --------------------------------------------
+// Passes over a transform of M elements in shared memory by T = M / E threads
+// (E = 12 or 4 elements per thread); the forward transforms of direct plans
+// (Dims::direct) run the radices in reverse order.
+
+// Reduction words of the CTA's transforms, zeroed by their first users: the
+// largest high word of the input, the sum of its magnitudes, and the same of
+// a second transform of the row (x-pass).
+constexpr int kFxWords = 1024;
+__device__ __forceinline__ int* fx_words() {
+    __shared__ int w[kFxWords];
+    return w;
+}
+// Maximum or sum over a transform into a zeroed word.  whole: the transform
+// owns whole warps (32 divides T).
+__device__ __forceinline__ void fx_reduce_max(int* word, int v, int lane, bool whole) {
+    if (whole) {
+        v = __reduce_max_sync(0xffffffffu, v);
+        if ((lane & 31) == 0) atomicMax(word, v);
+    } else {
+        atomicMax(word, v);
+    }
+}
+__device__ __forceinline__ void fx_reduce_add(int* word, unsigned v, int lane, bool whole) {
+    if (whole) {
+        v = __reduce_add_sync(0xffffffffu, v);
+        if ((lane & 31) == 0) atomicAdd((unsigned*)word, v);
+    } else {
+        atomicAdd((unsigned*)word, v);
+    }
+}
+__device__ __forceinline__ int fx_magnitude(double2 z) {
+    return max(fx_magnitude(__double2hiint(z.x)), fx_magnitude(__double2hiint(z.y)));
+}
+__device__ __forceinline__ fx2 fx_from(double2 z, int emax, int n0) {
+    return fx2{fx_from(__double2hiint(z.x), (unsigned)__double2loint(z.x), emax, n0),
+               fx_from(__double2hiint(z.y), (unsigned)__double2loint(z.y), emax, n0)};
+}
+__device__ __forceinline__ double2 fx_to(fx2 z, int eb) {
+    return make_double2(__longlong_as_double(fx_to(z.x, eb)), __longlong_as_double(fx_to(z.y, eb)));
+}
+__device__ __forceinline__ fx2 fx_ld(const longlong2* buf, int i) {
+    const longlong2 z = buf[i];
+    return fx2{z.x, z.y};
+}
+__device__ __forceinline__ void fx_st(longlong2* buf, int i, fx2 z) { buf[i] = make_longlong2(z.x, z.y); }
+
+// The exchange after a forward transform's first pass: radix-4 butterflies
+// store elements 4 j + r, a stride of four (4-way bank conflicts in eight
+// lanes), so that exchange goes through a permuted index that is
+// conflict-free for these stores and for the next pass's loads.  The
+// permutation stays within aligned blocks of 32 elements, so where T and M / 4
+// are multiples of 32 it is applied to the thread's lane.
+__device__ __forceinline__ bool swz_on(const Dims& d, int T) {
+    return (T & 31) == 0 && ((d.M / 4) & 31) == 0 && d.npass > 2 && d.radix[d.npass - 2] == 4;
+}
+__device__ __forceinline__ int swz(int i) { return i ^ ((i >> 3) & 3) ^ ((i >> 2) & 4); }
+// base of the four elements 4 j .. 4 j + 3 (element r at base ^ r)
+__device__ __forceinline__ int swz4(int j, bool on) { return on ? swz(4 * j) : 4 * j; }
+
+// The twiddled inputs of butterfly position k: r bits shifted out on the way.
+template <int R, bool INV>
+__device__ __forceinline__ void fx_twiddle(fx2* v, const FxTw* __restrict__ tab, int Ns, int k, int rsh) {
+    if (rsh) {
+        v[0].x = fx_round(v[0].x, rsh);
+        v[0].y = fx_round(v[0].y, rsh);
+    }
+#pragma unroll
+    for (int r = 1; r < R; ++r) {
+        const int4 w = __ldg(reinterpret_cast<const int4*>(tab + (r - 1) * Ns + k));
+        v[r] = fx_cmul<INV>(v[r], FxTw{w.x, w.y, w.z, w.w}, rsh);
+    }
+}
+template <int R, bool INV>
+__device__ __forceinline__ void fx_butterfly(fx2* v) {
+    if constexpr (R == 2) fx_bf2<INV>(v);
+    else if constexpr (R == 3) fx_bf3<INV>(v);
+    else fx_bf4<INV>(v);
+}
+
+// One pass after the first, in place (all loads, barrier, all stores,
+// barrier).  LAST: results rounded to FP64, eb their exponent base (fx_to).
+// lsw: the permutation of the lane for the loads (swz), or the lane.
+template <int E, int R, bool INV, bool LAST = false>
+__device__ __forceinline__ void fx_pass(longlong2* buf, int M, int Ns, unsigned mg, int lane, int T,
+                                        const FxTw* __restrict__ tab, int rsh, int lsw, int eb = 0) {
+    constexpr int NB = kFxNB<E, R>;
+    fx2 v[NB][R];
+    const int stride = M / R;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        if (fx_on<E, R>(lane + b * T, M)) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) v[b][r] = fx_ld(buf, lsw + b * T + r * stride);
+        }
+    }
     __syncthreads();
-    int Ns = 1;
-    for (int p = 0; p < d.npass; ++p) {
+    const ModNs mod(Ns, mg);
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const int j = lane + b * T;
+        if (!fx_on<E, R>(j, M)) continue;
+        const int k = mod(j);
+        fx_twiddle<R, INV>(v[b], tab, Ns, k, rsh);
+        fx_butterfly<R, INV>(v[b]);
+        const int base = (j - k) * R + k;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if constexpr (LAST) {
+                const double2 z = fx_to(v[b][r], eb);
+                buf[base + r * Ns] = make_longlong2(__double_as_longlong(z.x), __double_as_longlong(z.y));
+            } else {
+                fx_st(buf, base + r * Ns, v[b][r]);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// Passes 1 .. npass - 2 of a direct plan (INV) or of its mirror image (forward);
+// Ns and the bits shifted out so far are carried.
+template <int E, bool INV>
+__device__ __forceinline__ void fx_middle(longlong2* buf, const Dims& d, int lane, int T,
+                                          const FxTw* __restrict__ tab, float per, unsigned sum, float by_limit,
+                                          int& Ns, int& t) {
+    for (int p = 1; p < d.npass - 1; ++p) {
+        const int R = INV ? d.radix[p] : d.radix[d.npass - 1 - p];
+        const unsigned mg = INV ? d.mg[p] : d.mgf[p];
+        const FxTw* tp = tab + (INV ? d.twoff[p] : d.twofff[p]);
+        const int tn = max(t, fx_shift_total(Ns * R, per, sum, by_limit));
+        const int lsw = !INV && p == 1 && swz_on(d, T) ? swz(lane) : lane;
+        if (R == 4) fx_pass<E, 4, INV>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lsw);
+        else if (R == 2) fx_pass<E, 2, INV>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lane);
+        else fx_pass<E, 3, INV>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lane);
+        t = tn;
+        Ns *= R;
+    }
+}
+
+// ---- the general FP64 transform, FP64 in and out (fft_run) -----------------
+// First pass: the 12 elements of the thread from FP64, their common exponent
+// emax, the sum of magnitudes, a radix-R DFT without twiddles.  PRUNE: radix 3
+// with the middle input zero but for j = 0 (see fft_pass3_midzero).
+template <int R, bool INV, bool PRUNE>
+__device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg, int n0, int* words) {
+    constexpr int NB = kElemsPerThread / R;
+    double2 z[NB][R];
+    const int stride = M / R;
+    int mx = 0;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const int j = lane + b * Tg;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (PRUNE && r == 1 && (b > 0 || j > 0)) continue;
+            z[b][r] = reinterpret_cast<const double2*>(buf)[j + r * stride];
+            mx = max(mx, fx_magnitude(z[b][r]));
+        }
+    }
+    const bool whole = (Tg & 31) == 0;
+    fx_reduce_max(&words[0], mx, lane, whole);
+    __syncthreads();
+    const int emax = words[0] >> 20;
+    unsigned sum = 0;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+        const int j = lane + b * Tg;
+        fx2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            if (PRUNE && r == 1 && (b > 0 || j > 0)) continue;
+            v[r] = fx_from(z[b][r], emax, n0);
+            sum += fx_weight(v[r]);
+        }
+        if constexpr (PRUNE) {
+            if (b > 0 || j > 0) fx_bf3_bzero<INV>(v);
+            else fx_bf3<INV>(v);
+        } else {
+            fx_butterfly<R, INV>(v);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) fx_st(buf, j * R + r, v[r]);
+    }
+    fx_reduce_add(&words[512], sum, lane, whole);
+    __syncthreads();
+    return emax;
+}
+
+// The FP64 transform (see fft_run).  A transform with an infinity or NaN
+// gives NaN throughout.
+template <bool INV>
+__device__ __forceinline__ void fx_run(longlong2* buf, const Dims& d, int lane, const FxTw* __restrict__ tab) {
+    constexpr int E = kElemsPerThread;
+    int* words = fx_words() + ((int)threadIdx.x - lane);
+    if (lane == 0) {
+        words[0] = 0;
+        words[512] = 0;
+    }
+    __syncthreads();
+    const int R0 = d.radix[0];
+    const int n0 = R0 == 4 ? 4 : 3;
+    int emax;
+    if (INV && R0 == 3 && 3 * d.K == d.M) emax = fx_first<3, INV, INV>(buf, d.M, lane, d.Tg, n0, words);
+    else if (R0 == 3) emax = fx_first<3, INV, false>(buf, d.M, lane, d.Tg, n0, words);
+    else if (R0 == 4) emax = fx_first<4, INV, false>(buf, d.M, lane, d.Tg, n0, words);
+    else emax = fx_first<2, INV, false>(buf, d.M, lane, d.Tg, n0, words);
+    const unsigned sum = (unsigned)words[512];
+    const float per = fx_per(n0);
+    int Ns = R0, t = 0;
+    for (int p = 1; p < d.npass; ++p) {
+        const int R = d.radix[p];
+        const unsigned mg = d.mg[p];
+        const FxTw* tp = tab + d.twoff[p];
+        const int tn = max(t, fx_shift_total(Ns * R, per, sum, kFxByLimit));
+        const int rsh = tn - t;
+        t = tn;
+        if (p + 1 < d.npass) {
+            if (R == 4) fx_pass<E, 4, INV>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane);
+            else if (R == 2) fx_pass<E, 2, INV>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane);
+            else fx_pass<E, 3, INV>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane);
+        } else {
+            const int eb = fx_exponent_base(emax, n0, t);
+            if (R == 4) fx_pass<E, 4, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb);
+            else if (R == 2) fx_pass<E, 2, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb);
+            else fx_pass<E, 3, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb);
+        }
+        Ns *= R;
+    }
+}
+
+// FP32: passes [p0, p1) of the plan over the transform in buf.
+__device__ __forceinline__ const TwEnt<float>* f32_tab(const Dims& d, const float2* tw) {
+    return reinterpret_cast<const TwEnt<float>*>(reinterpret_cast<const char*>(tw) + d.tab_bytes);
+}
+template <int E, bool INV>
+__device__ __forceinline__ void f32_passes(float2* buf, const Dims& d, int lane, const float2* __restrict__ tw, int p0,
+                                           int p1) {
+    const TwEnt<float>* tab = f32_tab(d, tw);
+    int Ns = p0 == 0 ? 1 : d.radix[0];   // p0 is 0 or 1
+    for (int p = p0; p < p1; ++p) {
         const int R = d.radix[p];
         const int off = d.twoff[p];
         const unsigned mg = d.mg[p];
         if (INV && p == 0 && R == 3 && 3 * d.K == d.M) {
-            fft_pass3_midzero<INV>(buf, d.M, lane, d.Tg);
+            fft_pass3_midzero<E, INV>(buf, d.M, lane, d.Tg);
         } else if (R == 4) {
-            if (off >= 0) fft_pass4_fma<INV>(buf, d.M, Ns, mg, lane, d.Tg, tab + off);
-            else fft_pass<4, INV>(buf, d.M, Ns, mg, d.tstep[p], lane, d.Tg, tw);
+            if (off >= 0) fft_pass4_fma<E, INV>(buf, d.M, Ns, mg, lane, d.Tg, tab + off);
+            else fft_pass<E, 4, INV>(buf, d.M, Ns, mg, d.tstep[p], lane, d.Tg, tw);
         } else if (R == 2) {
-            if (off >= 0) fft_pass2_fma<INV>(buf, d.M, Ns, mg, lane, d.Tg, tab + off);
-            else fft_pass<2, INV>(buf, d.M, Ns, mg, d.tstep[p], lane, d.Tg, tw);
+            if (off >= 0) fft_pass2_fma<E, INV>(buf, d.M, Ns, mg, lane, d.Tg, tab + off);
+            else fft_pass<E, 2, INV>(buf, d.M, Ns, mg, d.tstep[p], lane, d.Tg, tw);
         } else {
-            fft_pass<3, INV>(buf, d.M, Ns, mg, d.tstep[p], lane, d.Tg, tw);
+            fft_pass<E, 3, INV>(buf, d.M, Ns, mg, d.tstep[p], lane, d.Tg, tw);
         }
         Ns *= R;
+    }
+}
+
+// Full transform: unnormalised, sign -1 (forward) or +1 (INV).  Every thread
+// of the CTA must call it (it synchronises the CTA); starts with a barrier so
+// that callers may fill buf just before.  tw points at the handle's twiddles
+// (Dims::twoff, tab_bytes).  Inverse transforms of truncated spectra (input
+// zero for K < n < M - K, K = M/3: the inverse transforms of this library)
+// take the pruned first radix-3 pass.
+template <bool INV, typename VT>
+__device__ __forceinline__ void fft_run(VT* buf, const Dims& d, int lane, const VT* __restrict__ tw) {
+    using T = decltype(buf[0].x);
+    if constexpr (sizeof(T) == 8) {
+        fx_run<INV>(reinterpret_cast<longlong2*>(buf), d, lane, reinterpret_cast<const FxTw*>(tw));
+    } else {
+        __syncthreads();
+        f32_passes<kElemsPerThread, INV>(buf, d, lane, tw, 0, d.npass);
     }
 }
 

@@ -17,17 +17,21 @@
 #include <stdint.h>
 
 #include "s2d.h"
+#include "s2d_fixed.cuh"
 
 namespace s2d {
 
 constexpr int kMaxPasses = 16;
 constexpr int kElemsPerThread = 12;   // FFT elements held per thread per pass
+// shared memory kept for the kernels' static arrays (the FP64 transforms'
+// reduction words, 4 KB, and the reductions of the diagnostics)
+constexpr int kStaticSmem = 1024 + 4096;
 // the FP32 x-pass with register radix-12/16 passes (s2d_xpass32.cuh): row
 // length and its padded shared-memory buffer (elements)
 constexpr int kX32M = 3072;
 constexpr int kX32Buf = kX32M + kX32M / 16;
 
-// Twiddles of one butterfly of a radix-4 (or radix-2) pass in FMA form:
+// FP32: twiddles of one butterfly of a radix-4 (or radix-2) pass in FMA form:
 // w_r = i^q_r * c_r * (1 + i t_r) with |t_r| <= 1, so that x*w_r costs two
 // FMAs on (x*i^q_r) and the scale c_r is folded into the butterfly's
 // additions (t0 = a + c2*C, E = B + (c3/c1)*D, y = t + c1*E ...).
@@ -38,6 +42,15 @@ struct __align__(16) TwEnt {
     T c1, c2, r31;  // c_1, c_2, c_3 / c_1
     int q;
     int pad;
+};
+
+template <typename T>
+struct TwTab {
+    using t = TwEnt<float>;
+};
+template <>
+struct TwTab<double> {
+    using t = FxTw;
 };
 
 // Geometry and FFT plan shared by every kernel of one handle.
@@ -51,14 +64,23 @@ struct Dims {
     int Tg;     // threads per transform = M / kElemsPerThread
     int npass;  // FFT passes
     int radix[kMaxPasses];
-    // per pass: offset (entries) of its TwEnt block, -1 if the pass uses the
-    // plain complex table (first pass, or a radix-3 pass after the first)
+    // per pass: offset (entries) of its block of per-pass twiddles.  FP32:
+    // TwEnt blocks, -1 if the pass uses the plain complex table (first pass,
+    // or a radix-3 pass after the first).  FP64: FxTw blocks of every pass
+    // after the first, w_1 of all Ns positions, then w_2, ...
     int twoff[kMaxPasses];
-    long long tab_bytes;  // byte offset of the TwEnt table after the complex table
+    long long tab_bytes;  // byte offset of those blocks (FP32: after the complex table; FP64: 0)
     // per pass, with Ns the product of the earlier radices: ceil(2^32 / Ns)
     // (0 for Ns = 1), for j mod Ns by a multiply-high, and M / (Ns R)
     unsigned mg[kMaxPasses];
     int tstep[kMaxPasses];
+    // direct: the plan's first radix is 3 and its last is 4, as the step's
+    // kernels of s2d_fxstep.cuh and s2d_f32step.cuh take it.  FP64: the step's
+    // forward transforms then run the radices in reverse order (radix[npass -
+    // 1] first), with their own constants
+    int direct;
+    unsigned mgf[kMaxPasses];
+    int twofff[kMaxPasses];
     // slabs of a decomposed run (s2d_slab.cu); a whole run has rows = M and
     // kx0 = 0.  rows: physical rows the x-pass processes.  kx0: true kx of
     // column 0 of the arrays a kernel is handed (a slab's column view: KX
@@ -80,6 +102,12 @@ inline void set_pass_constants(Dims* d) {
         d->tstep[p] = d->M / (ns * d->radix[p]);
         ns *= d->radix[p];
     }
+    ns = 1;
+    for (int p = 0; p < d->npass; ++p) {
+        d->mgf[p] = ns > 1 ? 0xFFFFFFFFu / (unsigned)ns + 1u : 0u;
+        ns *= d->radix[d->npass - 1 - p];
+    }
+    d->direct = d->radix[0] == 3 && d->radix[d->npass - 1] == 4;
 }
 
 // Terms of dW beyond the reference's (drag and a Kolmogorov source).
@@ -284,6 +312,10 @@ struct s2d_handle {
     bool pageable_direct = false;
     bool io_copy_only = false;   // S2D_HOST_IO=copy: every host array through copies
     s2d::Launch L_yinv, L_xpass, L_yfwd, L_xrow, L_ystore, L_ycol;
+    // small grids: the RK3 step's three kernels with 4 instead of 12 elements
+    // per thread (Dims::Tg = M / 4), K3 in one launch
+    bool small = false;
+    s2d::Launch S_yinv, S_xrow, S_yfwd, S_ystore;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     double graph_dt = 0.0;

@@ -23,6 +23,8 @@
 //
 // omega is not round-tripped through physical space (the reference does at
 // :435/:453); that changes omega by round-off only.
+#include "s2d_f32step.cuh"
+#include "s2d_fxstep.cuh"
 #include "s2d_step.cuh"
 
 #include <cuda_runtime.h>
@@ -100,8 +102,8 @@ __global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<T, B>)) k_yfwd_rk3
 
 // K3 split in two (FP64 single runs): forward y-FFT of one field's columns
 // into a compact array, then the epilogue of every mode.
-template <typename T, int B>
-__global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<T, B>))
+template <typename T>
+__global__ void __launch_bounds__(512)
     k_yfwd_col(Dims d, const typename Vec<T>::t* __restrict__ Iu, const typename Vec<T>::t* __restrict__ Iv,
                typename Vec<T>::t* Fu, typename Vec<T>::t* Fv, const typename Vec<T>::t* __restrict__ tw, int G) {
     using VT = typename Vec<T>::t;
@@ -119,6 +121,78 @@ __global__ void __launch_bounds__(256) k_stage(Dims d, const typename Vec<T>::t*
                                                const double* __restrict__ vk) {
     pdl_enter();
     if (stage_body<T>(d, Fu, Fv, S0, S1, Sdw, src, stage, dt, ph, cc, vk)) atomicOr(flags, 1u);
+}
+
+// ---- FP64, direct plans (s2d_fxstep.cuh) ---------------------------------
+// E elements per thread: 12, or 4 for small grids.  CTAs of at most 256
+// threads: three per SM (80 registers); up to 512: one.
+template <int E, int B>
+__global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<double, B>))
+    k_fx_yinv(Dims d, const double2* __restrict__ S, const double* __restrict__ rk2, FieldSet fs,
+              const FxTw* __restrict__ tw, int G) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    fx_yinv_body<E>(d, S, rk2, fs, tw, G, blockIdx.x, reinterpret_cast<double2*>(smem_raw));
+}
+
+template <int E, int B>
+__global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<double, B>))
+    k_fx_xpass(Dims d, double2* Iu, double2* Iv, const FxTw* __restrict__ tw, int G, double scale) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    fx_xpass_body<E>(d, Iu, Iv, tw, G, scale, blockIdx.x, reinterpret_cast<double2*>(smem_raw));
+}
+
+template <int E, int B>
+__global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<double, B>))
+    k_fx_yfwd_col(Dims d, const double2* __restrict__ Iu, const double2* __restrict__ Iv, double2* Fu, double2* Fv,
+                  const FxTw* __restrict__ tw, int G) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    fx_yfwd_col_body<E>(d, Iu, Iv, Fu, Fv, tw, G, blockIdx.x, reinterpret_cast<double2*>(smem_raw));
+}
+
+template <int E>
+__global__ void __launch_bounds__(512)
+    k_fx_yfwd_rk3(Dims d, const double2* __restrict__ Iu, const double2* __restrict__ Iv, double2* S0, double2* S1,
+                  double2* Sdw, const double2* __restrict__ src, int stage, double dt, Phys ph,
+                  const FxTw* __restrict__ tw, int G, unsigned int* flags) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    const bool bad = fx_yfwd_body<E>(d, Iu, Iv, S0, S1, Sdw, src, stage, dt, ph, tw, G, blockIdx.x,
+                                     reinterpret_cast<double2*>(smem_raw));
+    if (bad && flags) atomicOr(flags, 1u);
+}
+
+// ---- FP32, direct plans (s2d_f32step.cuh): CTAs of at most 256 threads four
+// per SM, of up to 512 two (64 registers).
+template <int E, int B>
+__global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<float, B>))
+    k_f32_yinv(Dims d, const float2* __restrict__ S, const double* __restrict__ rk2, FieldSet fs,
+               const float2* __restrict__ tw, int G) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    f32_yinv_body<E>(d, S, rk2, fs, tw, G, blockIdx.x, reinterpret_cast<float2*>(smem_raw));
+}
+
+template <int E, int B>
+__global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<float, B>))
+    k_f32_xpass(Dims d, float2* Iu, float2* Iv, const float2* __restrict__ tw, int G, float scale) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    f32_xpass_body<E>(d, Iu, Iv, tw, G, scale, blockIdx.x, reinterpret_cast<float2*>(smem_raw));
+}
+
+template <int E, int B>
+__global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<float, B>))
+    k_f32_yfwd_rk3(Dims d, const float2* __restrict__ Iu, const float2* __restrict__ Iv, float2* S0, float2* S1,
+                   float2* Sdw, const float2* __restrict__ src, int stage, double dt, Phys ph,
+                   const float2* __restrict__ tw, int G, unsigned int* flags) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    const bool bad = f32_yfwd_body<E>(d, Iu, Iv, S0, S1, Sdw, src, stage, dt, ph, tw, G, blockIdx.x,
+                                      reinterpret_cast<float2*>(smem_raw));
+    if (bad && flags) atomicOr(flags, 1u);
 }
 
 // ------------------------------------------------------------------------
@@ -640,13 +714,20 @@ cudaError_t Kern<T>::yinv(const Dims& d, const void* S, const double* rk2, const
     const int nb = ncg * fs.nf;
     const VT* s = (const VT*)S;
     const VT* t = (const VT*)tw;
-    switch (budget<T>(L.threads)) {
-        case 1: return launch_k(k_yinv<T, 1>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
-        case 2:
-            if constexpr (sizeof(T) == 4)
-                return launch_k(k_yinv<T, 2>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
-            return cudaErrorInvalidConfiguration;
-        default: return launch_k(k_yinv<T, 0>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
+    if constexpr (sizeof(T) == 8) {
+        const FxTw* ft = (const FxTw*)tw;
+        if (!d.direct) return launch_k(k_yinv<T, 0>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
+        if (d.Tg * 4 == d.M)
+            return L.threads <= 256 ? launch_k(k_fx_yinv<4, 1>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G)
+                                    : launch_k(k_fx_yinv<4, 0>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G);
+        return L.threads <= 256 ? launch_k(k_fx_yinv<12, 1>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G)
+                                : launch_k(k_fx_yinv<12, 0>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G);
+    } else {
+        if (!d.direct) return launch_k(k_yinv<T, 2>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
+        const bool four = d.Tg * 4 == d.M;
+        return launch_k(L.threads <= 256 ? (four ? k_f32_yinv<4, 1> : k_f32_yinv<12, 1>)
+                                         : (four ? k_f32_yinv<4, 2> : k_f32_yinv<12, 2>),
+                        nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
     }
 }
 
@@ -672,13 +753,20 @@ cudaError_t Kern<T>::xpass_bas(const Dims& d, void* Iu, void* Iv, const void* tw
     if constexpr (sizeof(T) == 4)
         if (d.M == kX32M && prescaled && !d.xgen)
             return launch_k(k_xpass32, d.rows, 256, 0, st, L.pdl, d, (float2*)Iu, (float2*)Iv, (const float2*)tw);
-    switch (budget<T>(L.threads)) {
-        case 1: return launch_k(k_xpass_bas<T, 1>, nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
-        case 2:
-            if constexpr (sizeof(T) == 4)
-                return launch_k(k_xpass_bas<T, 2>, nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
-            return cudaErrorInvalidConfiguration;
-        default: return launch_k(k_xpass_bas<T, 0>, nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
+    if constexpr (sizeof(T) == 8) {
+        const FxTw* ft = (const FxTw*)tw;
+        if (!d.direct) return launch_k(k_xpass_bas<T, 0>, nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
+        if (d.Tg * 4 == d.M)
+            return L.threads <= 256 ? launch_k(k_fx_xpass<4, 1>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale)
+                                    : launch_k(k_fx_xpass<4, 0>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale);
+        return L.threads <= 256 ? launch_k(k_fx_xpass<12, 1>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale)
+                                : launch_k(k_fx_xpass<12, 0>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale);
+    } else {
+        if (!d.direct) return launch_k(k_xpass_bas<T, 2>, nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
+        const bool four = d.Tg * 4 == d.M;
+        return launch_k(L.threads <= 256 ? (four ? k_f32_xpass<4, 1> : k_f32_xpass<12, 1>)
+                                         : (four ? k_f32_xpass<4, 2> : k_f32_xpass<12, 2>),
+                        nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
     }
 }
 
@@ -691,9 +779,18 @@ cudaError_t Kern<T>::yfwd_rk3(const Dims& d, const void* Iu, const void* Iv, voi
     // FP32 CTAs of up to 256 threads at 64 registers, four per SM (at 80
     // registers, three per SM: 0.244 against 0.219 ms of K3 per 2048^2 step)
     if constexpr (sizeof(T) == 4)
-        if (L.threads <= 256)
-            return launch_k(k_yfwd_rk3<T, 1>, nb, L.threads, L.smem, st, L.pdl, d, (const VT*)Iu, (const VT*)Iv,
-                            (VT*)S0, (VT*)S1, (VT*)Sdw, (const VT*)src, stage, dt, ph, (const VT*)tw, L.G, flags);
+        if (d.direct) {
+            const bool four = d.Tg * 4 == d.M;
+            return launch_k(L.threads <= 256 ? (four ? k_f32_yfwd_rk3<4, 1> : k_f32_yfwd_rk3<12, 1>)
+                                             : (four ? k_f32_yfwd_rk3<4, 2> : k_f32_yfwd_rk3<12, 2>),
+                            nb, L.threads, L.smem, st, L.pdl, d, (const VT*)Iu, (const VT*)Iv, (VT*)S0, (VT*)S1,
+                            (VT*)Sdw, (const VT*)src, stage, dt, ph, (const VT*)tw, L.G, flags);
+        }
+    if constexpr (sizeof(T) == 8)
+        if (d.direct)
+            return launch_k(d.Tg * 4 == d.M ? k_fx_yfwd_rk3<4> : k_fx_yfwd_rk3<12>, nb, L.threads, L.smem, st, L.pdl, d,
+                            (const VT*)Iu, (const VT*)Iv, (VT*)S0, (VT*)S1, (VT*)Sdw, (const VT*)src, stage, dt, ph,
+                            (const FxTw*)tw, L.G, flags);
     return launch_k(k_yfwd_rk3<T, 0>, nb, L.threads, L.smem, st, L.pdl, d, (const VT*)Iu, (const VT*)Iv, (VT*)S0,
                     (VT*)S1, (VT*)Sdw, (const VT*)src, stage, dt, ph, (const VT*)tw, L.G, flags);
 }
@@ -705,20 +802,17 @@ cudaError_t Kern<T>::yfwd_col(const Dims& d, const void* Iu, const void* Iv, voi
     const int ncg = (d.KX + L.G - 1) / L.G;
     const VT* u = (const VT*)Iu;
     const VT* v = (const VT*)Iv;
-    const VT* t = (const VT*)tw;
-    switch (budget<T>(L.threads)) {
-        case 1:
-            return launch_k(k_yfwd_col<T, 1>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v, (VT*)Fu, (VT*)Fv, t,
-                            L.G);
-        case 2:
-            if constexpr (sizeof(T) == 4)
-                return launch_k(k_yfwd_col<T, 2>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v, (VT*)Fu,
-                                (VT*)Fv, t, L.G);
-            return cudaErrorInvalidConfiguration;
-        default:
-            return launch_k(k_yfwd_col<T, 0>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v, (VT*)Fu, (VT*)Fv, t,
-                            L.G);
+    if constexpr (sizeof(T) == 8) {   // FP64 runs alone split their K3
+        const FxTw* ft = (const FxTw*)tw;
+        if (d.direct)
+            return L.threads <= 256 ? launch_k(k_fx_yfwd_col<12, 1>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v,
+                                               (VT*)Fu, (VT*)Fv, ft, L.G)
+                                    : launch_k(k_fx_yfwd_col<12, 0>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v,
+                                               (VT*)Fu, (VT*)Fv, ft, L.G);
+        return launch_k(k_yfwd_col<T>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v, (VT*)Fu, (VT*)Fv,
+                        (const VT*)tw, L.G);
     }
+    return cudaErrorInvalidConfiguration;
 }
 
 template <typename T>
@@ -869,26 +963,39 @@ cudaError_t configure_kernels(int max_smem_optin) {
         cudaError_t e2 = set_smem(k, max_smem_optin);       \
         if (e2 != cudaSuccess && e == cudaSuccess) e = e2;  \
     } while (0)
-    S2D_SET((k_yinv<double, 1>));
+    S2D_SET((k_f32_yinv<12, 1>));
+    S2D_SET((k_f32_yinv<12, 2>));
+    S2D_SET((k_f32_yinv<4, 1>));
+    S2D_SET((k_f32_yinv<4, 2>));
+    S2D_SET((k_f32_xpass<12, 1>));
+    S2D_SET((k_f32_xpass<12, 2>));
+    S2D_SET((k_f32_xpass<4, 1>));
+    S2D_SET((k_f32_xpass<4, 2>));
+    S2D_SET((k_f32_yfwd_rk3<12, 1>));
+    S2D_SET((k_f32_yfwd_rk3<12, 2>));
+    S2D_SET((k_f32_yfwd_rk3<4, 1>));
+    S2D_SET((k_f32_yfwd_rk3<4, 2>));
+    S2D_SET((k_fx_yinv<12, 1>));
+    S2D_SET((k_fx_yinv<12, 0>));
+    S2D_SET((k_fx_yinv<4, 1>));
+    S2D_SET((k_fx_yinv<4, 0>));
+    S2D_SET((k_fx_xpass<12, 1>));
+    S2D_SET((k_fx_xpass<12, 0>));
+    S2D_SET((k_fx_xpass<4, 1>));
+    S2D_SET((k_fx_xpass<4, 0>));
+    S2D_SET((k_fx_yfwd_col<12, 1>));
+    S2D_SET((k_fx_yfwd_col<12, 0>));
+    S2D_SET(k_fx_yfwd_rk3<12>);
+    S2D_SET(k_fx_yfwd_rk3<4>);
     S2D_SET((k_yinv<double, 0>));
-    S2D_SET((k_yinv<float, 1>));
     S2D_SET((k_yinv<float, 2>));
-    S2D_SET((k_yinv<float, 0>));
     S2D_SET(k_xpass_rhs<double>);
     S2D_SET(k_xpass_rhs<float>);
-    S2D_SET((k_xpass_bas<double, 1>));
     S2D_SET((k_xpass_bas<double, 0>));
-    S2D_SET((k_xpass_bas<float, 1>));
     S2D_SET((k_xpass_bas<float, 2>));
-    S2D_SET((k_xpass_bas<float, 0>));
-    S2D_SET((k_yfwd_col<double, 1>));
-    S2D_SET((k_yfwd_col<double, 0>));
-    S2D_SET((k_yfwd_col<float, 1>));
-    S2D_SET((k_yfwd_col<float, 2>));
-    S2D_SET((k_yfwd_col<float, 0>));
+    S2D_SET(k_yfwd_col<double>);
     S2D_SET((k_yfwd_rk3<double, 0>));
     S2D_SET((k_yfwd_rk3<float, 0>));
-    S2D_SET((k_yfwd_rk3<float, 1>));
     S2D_SET(k_xinv_cfl<double>);
     S2D_SET(k_xinv_moments<double>);
     S2D_SET(k_xinv_moments<float>);

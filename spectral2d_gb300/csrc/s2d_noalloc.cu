@@ -38,15 +38,14 @@ struct DevState {
     bool ready;              // symbol address resolved for this device
     unsigned char* base;     // device address of g_s2d_noalloc_scratch
     int tables_nx;           // nx whose twiddle and 1/k^2 tables are resident (0: none)
-    int ntab;                // FMA-form twiddle entries of that plan
+    int ntab;                // twiddle entries of that plan
     Dims plan;               // that plan (radices, pass constants, table offsets)
     int max_smem;
 };
 DevState g_dev[kMaxDevices];
 
 // static host staging for the twiddle tables (no heap)
-double g_host_tw[2 * kMaxM];
-TwEnt<double> g_host_tab[kMaxM];
+FxTw g_host_tab[2 * kMaxM];
 
 // The status code is the only error report: writing a message would need
 // the library's message buffer, whose update may allocate.
@@ -66,11 +65,11 @@ bool plan_noalloc(int nx, Dims* d) {
     if (!factor_plan(d->M, d)) return false;
     d->Tg = d->M / kElemsPerThread;
     d->rows = d->M;
-    d->tab_bytes = (long long)up256((size_t)d->M * sizeof(double2));
+    d->tab_bytes = 0;
     return true;
 }
 
-// Carve the scratch array: twiddles (+ FMA blocks) | rk2 | S | Sdw | I0 | I1.
+// Carve the scratch array: twiddle blocks | rk2 | S | Sdw | I0 | I1.
 struct Carve {
     size_t tw, rk2, S, Sdw, I0, I1, end;
 };
@@ -79,7 +78,7 @@ Carve carve(const Dims& d, int ntab) {
     Carve c{};
     const size_t state = (size_t)d.KX * d.ldS * sizeof(double2);
     const size_t inter = (size_t)d.M * d.ldI * sizeof(double2);
-    const size_t twb = up256((size_t)d.M * sizeof(double2)) + (size_t)ntab * sizeof(TwEnt<double>);
+    const size_t twb = (size_t)ntab * sizeof(FxTw);
     c.tw = 0;
     c.rk2 = c.tw + up256(twb);
     c.S = c.rk2 + up256((size_t)d.KX * d.ldS * sizeof(double));
@@ -125,7 +124,7 @@ S2D_API int s2d_compute_rhs_noalloc(int32_t nx, double nu, const double* wC_dev,
         int optin = 0;
         if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
             return err(S2D_ERR_CUDA, "cudaDeviceGetAttribute failed");
-        ds.max_smem = optin - 1024;
+        ds.max_smem = optin - kStaticSmem;
         if (configure_kernels(ds.max_smem) != cudaSuccess) return err(S2D_ERR_CUDA, "cudaFuncSetAttribute failed");
         ds.base = (unsigned char*)p;
         ds.tables_nx = 0;
@@ -139,18 +138,15 @@ S2D_API int s2d_compute_rhs_noalloc(int32_t nx, double nu, const double* wC_dev,
         ntab = ds.ntab;
     } else {
         if (!plan_noalloc(nx, &d)) return err(S2D_ERR_UNSUPPORTED, "padded grid is not 2^a 3^b");
-        ntab = fill_fma_tables<double>(&d, g_host_tab, kMaxM);
+        ntab = fill_tables<double>(&d, g_host_tab, 2 * kMaxM);
         if (ntab < 0) return err(S2D_ERR_INVALID, "twiddle table exceeds its static buffer");
         if (carve(d, ntab).end > S2D_NOALLOC_SCRATCH_BYTES)
             return err(S2D_ERR_INVALID, "grid does not fit the static scratch");
-        fill_twiddles(d.M, g_host_tw);
         const Carve c0 = carve(d, ntab);
         ds.tables_nx = 0;   // until the new tables are queued
         // the copies are queued on st before any kernel of this call that reads them
-        if (cudaMemcpyAsync(B + c0.tw, g_host_tw, (size_t)d.M * sizeof(double2), cudaMemcpyHostToDevice, st) !=
-                cudaSuccess ||
-            (ntab > 0 && cudaMemcpyAsync(B + c0.tw + d.tab_bytes, g_host_tab, (size_t)ntab * sizeof(TwEnt<double>),
-                                         cudaMemcpyHostToDevice, st) != cudaSuccess))
+        if (cudaMemcpyAsync(B + c0.tw, g_host_tab, (size_t)ntab * sizeof(FxTw), cudaMemcpyHostToDevice, st) !=
+            cudaSuccess)
             return err(S2D_ERR_CUDA, "twiddle upload failed");
         // pageable source buffers: the copies have read them when cudaMemcpyAsync returns
         if (Kern<double>::init_rk2(d, (double*)(B + c0.rk2), st) != cudaSuccess)

@@ -13,7 +13,7 @@ namespace s2d {
 
 // exp(-2 pi i r / M) correctly rounded in practice: octant reduction with
 // exact integer arithmetic, residual angle in [0, pi/4] in long double.
-inline void twiddle(long long r, long long M, double* c, double* s) {
+inline void twiddle_ld(long long r, long long M, long double* c, long double* s) {
     const long double PI_4 = 0.785398163397448309615660845819875721L;
     r %= M;
     const long long n8 = 8 * r;
@@ -32,8 +32,14 @@ inline void twiddle(long long r, long long M, double* c, double* s) {
         case 6: C = sx; S = -cx; break;
         default: C = cx; S = -sx; break;
     }
+    *c = C;
+    *s = -S;  // forward sign
+}
+inline void twiddle(long long r, long long M, double* c, double* s) {
+    long double C, S;
+    twiddle_ld(r, M, &C, &S);
     *c = (double)C;
-    *s = -(double)S;  // forward sign
+    *s = (double)S;
 }
 
 // exp(-2 pi i m / M) = i^q * c * (1 + i t) with |t| <= 1 (needs 4 | M):
@@ -89,52 +95,79 @@ inline bool factor_plan(int M, Dims* d, int plan = 0) {
     return true;
 }
 
-// Entries of the FMA-form twiddle blocks of a plan: one per butterfly
-// position k < Ns of every radix-4 or radix-2 pass after the first.
-inline int fma_table_entries(const Dims& d) {
-    int n = 0, Ns = 1;
+// Entries of the per-pass twiddle blocks of a plan (Dims::twoff): FP32 one
+// TwEnt per butterfly position k < Ns of every radix-4 or radix-2 pass after
+// the first; FP64 R - 1 factors per position of every pass after the first,
+// and the same for the mirrored order.
+template <typename T>
+inline int table_entries(const Dims& d) {
+    int n = 0, Ns = 1, Nm = 1;
     for (int p = 0; p < d.npass; ++p) {
-        if (p > 0 && (d.radix[p] == 4 || d.radix[p] == 2)) n += Ns;
+        const int Rm = d.radix[d.npass - 1 - p];
+        if (p > 0) {
+            if (sizeof(T) == 8) n += Ns * (d.radix[p] - 1) + (d.direct ? Nm * (Rm - 1) : 0);
+            else if (d.radix[p] == 4 || d.radix[p] == 2) n += Ns;
+        }
         Ns *= d.radix[p];
+        Nm *= Rm;
     }
     return n;
 }
 
-// The FMA-form twiddle blocks (TwEnt) of every radix-4/2 pass after the
-// first, written to out[0 .. fma_table_entries(*d)), and each pass's offset
-// into them in d->twoff (-1 for passes that use the plain complex table).
+// exp(-2 pi i m / M) in units of 2^-62.
+inline FxTw twiddle_fixed(long long m, long long M) {
+    long double c, s;
+    twiddle_ld(m, M, &c, &s);
+    return fx_limbs(llrintl(ldexpl(c, kFxOne)), llrintl(ldexpl(s, kFxOne)));
+}
+
+// The per-pass twiddle blocks, written to out[0 .. table_entries<T>(*d)), and
+// each pass's offset into them in d->twoff (-1 for passes without one).
 // Returns the entry count, or -1 if it exceeds cap (nothing is written then).
 template <typename T>
-inline int fill_fma_tables(Dims* d, TwEnt<T>* out, int cap) {
-    if (fma_table_entries(*d) > cap) return -1;
-    int n = 0, Ns = 1;
+inline int fill_tables(Dims* d, typename TwTab<T>::t* out, int cap) {
+    if (table_entries<T>(*d) > cap) return -1;
+    int n = 0, Ns = 1, Nm = 1;
     for (int p = 0; p < d->npass; ++p) {
-        const int R = d->radix[p];
-        d->twoff[p] = -1;
-        if (p > 0 && (R == 4 || R == 2)) {
+        const int R = d->radix[p], Rm = d->radix[d->npass - 1 - p];
+        const long long step = d->M / (Ns * R);
+        d->twoff[p] = d->twofff[p] = -1;
+        if constexpr (sizeof(T) == 8) {
+            if (p > 0) {
+                d->twoff[p] = n;
+                for (int r = 1; r < R; ++r)
+                    for (int k = 0; k < Ns; ++k) out[n++] = twiddle_fixed((long long)r * k * step, d->M);
+                if (d->direct) {
+                    d->twofff[p] = n;
+                    for (int r = 1; r < Rm; ++r)
+                        for (int k = 0; k < Nm; ++k)
+                            out[n++] = twiddle_fixed((long long)r * k * (d->M / (Nm * Rm)), d->M);
+                }
+            }
+        } else if (p > 0 && (R == 4 || R == 2)) {
             d->twoff[p] = n;
-            const long long step = d->M / (Ns * R);
             for (int k = 0; k < Ns; ++k) {
-                TwEnt<T> e{};
+                TwEnt<float> e{};
                 int qs[4] = {0, 0, 0, 0};
                 long double cs[4] = {1, 1, 1, 1}, ts[4] = {0, 0, 0, 0};
                 for (int r = 1; r < R; ++r) twiddle_fma((long long)r * k * step, d->M, &qs[r], &cs[r], &ts[r]);
-                e.t1 = (T)ts[1];
-                e.t2 = (T)ts[2];
-                e.t3 = (T)ts[3];
-                e.c1 = (T)cs[1];
-                e.c2 = (T)cs[2];
-                e.r31 = (T)(cs[3] / cs[1]);
+                e.t1 = (float)ts[1];
+                e.t2 = (float)ts[2];
+                e.t3 = (float)ts[3];
+                e.c1 = (float)cs[1];
+                e.c2 = (float)cs[2];
+                e.r31 = (float)(cs[3] / cs[1]);
                 e.q = qs[1] | (qs[2] << 2) | (qs[3] << 4);
                 out[n++] = e;
             }
         }
         Ns *= R;
+        Nm *= Rm;
     }
     return n;
 }
 
-// The plain complex twiddles exp(-2 pi i t / M), t < M, as (re, im) pairs.
+// The plain complex twiddles exp(-2 pi i t / M), t < M, as (re, im) pairs (FP32 handles).
 inline void fill_twiddles(int M, double* out2M) {
     for (int t = 0; t < M; ++t) twiddle(t, M, &out2M[2 * t], &out2M[2 * t + 1]);
 }
