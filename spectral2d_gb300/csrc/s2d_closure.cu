@@ -1258,25 +1258,38 @@ cudaError_t launch_wgrad(const __nv_bfloat16* dz, const __nv_bfloat16* in, float
                     err);
 }
 
-// out[i] = sum_b part[b * n + i], b in order.
+// out[i] = sum_b part[b * n + i], b in order; 16 loads in flight per thread,
+// small CTAs so that the 4 to 9 thousand sums spread over the SMs.
 __global__ void k_reduce_rows(const float* __restrict__ part, int nblk, long n, float* out) {
+    constexpr int U = 16;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         float s = 0.f;
-        for (int b = 0; b < nblk; ++b) s += part[(long)b * n + i];
+        for (int b0 = 0; b0 < nblk; b0 += U) {
+            float v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) v[u] = b0 + u < nblk ? part[(long)(b0 + u) * n + i] : 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (b0 + u < nblk) s += v[u];
+        }
         out[i] = s;
     }
 }
 
-// MSE loss: dz[p, 0] = 2 (y - t) / n, other channels 0; per-block loss sums.
+// MSE loss: dz[p, 0] = 2 (y - t) / n, channels 1 .. 15 zero; per-block loss
+// sums.  Memory-bound (40 bytes per pixel): a pixel's 32 bytes of dz go out as
+// two 16-byte stores, not sixteen 2-byte ones (64 x 192^2: 242 us that way).
+constexpr int kMseBlocks = 1024;
 __global__ void k_mse(const float* __restrict__ y, const float* __restrict__ tgt, long P, float inv_n,
-                      __nv_bfloat16* dz, int CO, double* part) {
+                      __nv_bfloat16* dz, double* part) {
     __shared__ double red[256];
     double s = 0.0;
     for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < P; p += (long)gridDim.x * blockDim.x) {
         const float e = y[p] - tgt[p];
         s += (double)e * e;
-        dz[p * CO] = __float2bfloat16_rn(2.f * e * inv_n);
-        for (int c = 1; c < CO; ++c) dz[p * CO + c] = __float2bfloat16_rn(0.f);
+        uint4* o = reinterpret_cast<uint4*>(dz + p * 16);
+        o[0] = make_uint4(pack_bf16(2.f * e * inv_n, 0.f), 0u, 0u, 0u);
+        o[1] = make_uint4(0u, 0u, 0u, 0u);
     }
     red[threadIdx.x] = s;
     __syncthreads();
@@ -1324,9 +1337,9 @@ __global__ void k_pack(const float* __restrict__ data, const float* __restrict__
         const long b = p / HW, q = p - b * HW;
         const float* s = data + ((long)idx[b] * HW + q) * 3;
         const float ia = amp ? 1.f / amp[idx[b]] : 1.f;
-        uint32_t* xr = reinterpret_cast<uint32_t*>(x + p * 16);
-        xr[0] = pack_bf16(s[0] * r0 * ia, s[1] * r1 * ia);
-        for (int c = 1; c < 8; ++c) xr[c] = 0u;
+        uint4* xr = reinterpret_cast<uint4*>(x + p * 16);
+        xr[0] = make_uint4(pack_bf16(s[0] * r0 * ia, s[1] * r1 * ia), 0u, 0u, 0u);
+        xr[1] = make_uint4(0u, 0u, 0u, 0u);
         if (tgt) tgt[p] = s[2] * r2 * ia * ia;
     }
 }
@@ -1877,8 +1890,8 @@ int forward(s2d_cnn* c, int B, bool keep_z, bool pdl = false) {
 // loss of the batch (targets in tgt) and, with grads, the full backward pass
 int loss_backward(s2d_cnn* c, int B, bool grads, double* loss) {
     const long P = (long)B * c->H * c->Wd;
-    const int lb = 256;
-    k_mse<<<lb, 256, 0, c->stream>>>(c->Y, c->tgt, P, 1.0f / (float)P, c->dZ6, 16, c->lpart);
+    const int lb = kMseBlocks;
+    k_mse<<<lb, 256, 0, c->stream>>>(c->Y, c->tgt, P, 1.0f / (float)P, c->dZ6, c->lpart);
     C_CUDA(cudaGetLastError());
     std::vector<double> lp(lb);
     C_CUDA(cudaMemcpyAsync(lp.data(), c->lpart, sizeof(double) * lb, cudaMemcpyDeviceToHost, c->stream));
@@ -1911,7 +1924,7 @@ int loss_backward(s2d_cnn* c, int B, bool grads, double* loss) {
                 else
                     C_CUDA((launch_wgrad<32, 32>(dz, in, c->part, B, c->H, c->Wd, g, c->cflags, c->stream, &nblk)));
             }
-            k_reduce_rows<<<nblocks(n, 256), 256, 0, c->stream>>>(c->part, nblk, n, c->grad + c->poff[l]);
+            k_reduce_rows<<<nblocks(n, 64), 64, 0, c->stream>>>(c->part, nblk, n, c->grad + c->poff[l]);
             C_CUDA(cudaGetLastError());
             if (l > 0) {
                 __nv_bfloat16* out = c->keep ? c->dZk[l - 1] : bufs[l & 1];
@@ -2261,7 +2274,7 @@ S2D_API int s2d_cnn_create(int32_t grid, int32_t max_batch, uint64_t seed, int32
               cudaMalloc(&c->Y, P * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&c->tgt, P * sizeof(float)) == cudaSuccess &&
               cudaMalloc(&c->part, c->part_n * sizeof(float)) == cudaSuccess &&
-              cudaMalloc(&c->lpart, 256 * sizeof(double)) == cudaSuccess &&
+              cudaMalloc(&c->lpart, kMseBlocks * sizeof(double)) == cudaSuccess &&
               cudaMalloc(&c->idx, max_batch * sizeof(int)) == cudaSuccess &&
               cudaMalloc(&c->sumsq, 64) == cudaSuccess && cudaMalloc(&c->cflags, 64) == cudaSuccess &&
               cudaMemset(c->cflags, 0, 64) == cudaSuccess;
