@@ -585,7 +585,7 @@ struct NetArgs {
     const float* bias[kLayers];
     __nv_bfloat16* act[2];             // framed 32-channel images
     float* y;                          // output channel 0, [B][H][Wd]
-    unsigned int* bar;                 // grid barrier: arrivals of this launch
+    unsigned int* bar;                 // grid barrier: arrivals of this launch, CTAs that left (zero between launches)
     unsigned int* err;
     int B, H, Wd;
     int stall;                         // fault injection: CTA 0 skips its first grid-barrier arrival
@@ -625,47 +625,27 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 }
 
 // Grid barrier of one thread per CTA (the CTA synchronised before and
-// after): *bar counts the arrivals of the launch (zeroed before it), the
+// after), arrival and wait apart: *bar counts the arrivals of the launch, the
 // j-th barrier opens at j * gridDim.x.  Bounded: false after a second.
-__device__ __forceinline__ bool net_grid_sync(unsigned int* bar, unsigned int target) {
+__device__ __forceinline__ void net_grid_arrive(unsigned int* bar) {
     __threadfence();
     atomicAdd(bar, 1u);
+}
+__device__ __forceinline__ bool net_grid_wait(const unsigned int* bar, unsigned int target) {
     const unsigned long long t0 = globaltimer_ns();
-    while (ld_acquire_u32(bar) < target) {
+    while (ld_acquire_u32(bar) < target)
         if (globaltimer_ns() - t0 > 1000000000ull) return false;
-        __nanosleep(64);
-    }
     return true;
 }
 
-// One layer over this CTA's tiles (tile blockIdx.x + k gridDim.x); irun is
-// the CTA's running tile count over all layers, which fixes every slot,
-// accumulator and barrier phase.
-template <int KC, int NC, bool LAST>
-__device__ __forceinline__ void net_layer(const CUtensorMap* tin, const __nv_bfloat16* __restrict__ W,
-                                          const float* __restrict__ bias, __nv_bfloat16* out, float* yout,
-                                          const NetArgs& a, NetShared& sh, unsigned char* gbase, uint32_t sbase,
-                                          int& irun) {
-    constexpr int KG = KC / 8;                 // 8-channel groups of a pixel
-    constexpr int ROWB = KC * 2;               // bytes of one pixel
-    constexpr int BOX = kNetBoxRows * kNetBoxW * ROWB;
-    constexpr int N = 3 * NC;                  // the MMA's columns: (dx, output channel)
-    constexpr int NG = N / 8;                  // 8-column groups
-    constexpr int CORE = 128;
-    constexpr int WGROUP = KG * CORE;          // 8 columns x all input channels
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int H = a.H, Wd = a.Wd;
-    const int tiles_x = (Wd + kNetOutW - 1) / kNetOutW;
-    const int tiles_img = tiles_x * ((H + kNetOutH - 1) / kNetOutH);
-    const int ntiles = tiles_img * a.B;
-    const int nk = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-    const uint32_t bw = sbase + kNetSlots * kNetSlotBytes;
-    volatile int* abort = &sh.abort;
-
-    // the layer's weights as the B operands of the three rows of taps: for
-    // row dy, column group g = (dx, 8 output channels), the input channels
-    // K-major in core matrices (the previous layer's MMAs are all complete)
-    for (int i = tid; i < 3 * N * KG; i += blockDim.x) {
+// A layer's weights as the B operands of the three rows of taps: for row dy,
+// column group g = (dx, 8 output channels), the input channels K-major in core
+// matrices; and its biases.  At most two 16-byte pieces per thread.
+template <int KC, int NC>
+__device__ __forceinline__ void net_stage_weights(const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
+                                                  NetShared& sh, unsigned char* gbase) {
+    constexpr int KG = KC / 8, N = 3 * NC, NG = N / 8, CORE = 128;
+    for (int i = threadIdx.x; i < 3 * N * KG; i += blockDim.x) {
         const int nl = i % 8;
         const int kg = (i / 8) % KG;
         const int g = (i / (8 * KG)) % NG;
@@ -677,11 +657,31 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, const __nv_bfl
         const int off = ((dyi * NG + g) * KG + kg) * CORE + nl * 16;
         *reinterpret_cast<uint4*>(gbase + kNetSlots * kNetSlotBytes + off) = v;
     }
-    if (tid < NC) sh.bias[tid] = bias[tid];
+    if ((int)threadIdx.x < NC) sh.bias[threadIdx.x] = bias[threadIdx.x];
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+}
+
+// One layer over this CTA's tiles (tile blockIdx.x + k gridDim.x), its weights
+// staged; irun is the CTA's running tile count over all layers, which fixes
+// every slot, accumulator and barrier phase.
+template <int KC, int NC, bool LAST>
+__device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16* out, float* yout, const NetArgs& a,
+                                          NetShared& sh, uint32_t sbase, int& irun) {
+    constexpr int KG = KC / 8;                 // 8-channel groups of a pixel
+    constexpr int ROWB = KC * 2;               // bytes of one pixel
+    constexpr int BOX = kNetBoxRows * kNetBoxW * ROWB;
+    constexpr int N = 3 * NC;                  // the MMA's columns: (dx, output channel)
+    constexpr int NG = N / 8;                  // 8-column groups
+    constexpr int CORE = 128;
+    constexpr int WGROUP = KG * CORE;          // 8 columns x all input channels
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int H = a.H, Wd = a.Wd;
+    const int tiles_x = (Wd + kNetOutW - 1) / kNetOutW;
+    const int tiles_img = tiles_x * ((H + kNetOutH - 1) / kNetOutH);
+    const int ntiles = tiles_img * a.B;
+    const int nk = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    const uint32_t bw = sbase + kNetSlots * kNetSlotBytes;
+    volatile int* abort = &sh.abort;
 
     // tile k: output rows [oy0, oy0 + 8), columns [ox0, ox0 + 14); its box is
     // image rows oy0 - 1 .. oy0 + 8 and columns ox0 - 1 .. ox0 + 14, at
@@ -888,37 +888,44 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_fwd(const __grid_constan
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
         sh.abort = 0;
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-
     int irun = 0, nbar = 0;
-    auto barrier = [&]() {
+    // Between layers: every CTA arrives once its tiles are stored, stages the
+    // next layer's weights while the others arrive (its own MMAs, the readers
+    // of the old ones, are complete), then waits.
+    auto before_layer = [&](auto stage, bool first) {
         __syncthreads();
-        ++nbar;
+        nbar += first ? 0 : 1;
         const bool skip = a.stall && nbar == 1 && blockIdx.x == 0;   // host-injected fault (tests)
-        if (tid == 0 && !sh.abort && !skip && !net_grid_sync(a.bar, (unsigned int)nbar * gridDim.x)) {
+        const bool sync = !first && tid == 0 && !sh.abort && !skip;
+        if (sync) net_grid_arrive(a.bar);
+        stage();
+        if (sync && !net_grid_wait(a.bar, (unsigned int)nbar * gridDim.x)) {
             sh.abort = 1;
             atomicOr(a.err, 4u);
         }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
         __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     };
-    net_layer<16, 32, false>(&m_in, a.W[0], a.bias[0], a.act[0], nullptr, a, sh, gbase, sbase, irun);
-    barrier();
-    net_layer<32, 32, false>(&m_a0, a.W[1], a.bias[1], a.act[1], nullptr, a, sh, gbase, sbase, irun);
-    barrier();
-    net_layer<32, 32, false>(&m_a1, a.W[2], a.bias[2], a.act[0], nullptr, a, sh, gbase, sbase, irun);
-    barrier();
-    net_layer<32, 32, false>(&m_a0, a.W[3], a.bias[3], a.act[1], nullptr, a, sh, gbase, sbase, irun);
-    barrier();
-    net_layer<32, 32, false>(&m_a1, a.W[4], a.bias[4], a.act[0], nullptr, a, sh, gbase, sbase, irun);
-    barrier();
-    net_layer<32, 16, true>(&m_a0, a.W[5], a.bias[5], nullptr, a.y, a, sh, gbase, sbase, irun);
+    before_layer([&] { net_stage_weights<16, 32>(a.W[0], a.bias[0], sh, gbase); }, true);
+    net_layer<16, 32, false>(&m_in, a.act[0], nullptr, a, sh, sbase, irun);
+#pragma unroll 1
+    for (int l = 1; l < kLayers - 1; ++l) {
+        before_layer([&] { net_stage_weights<32, 32>(a.W[l], a.bias[l], sh, gbase); }, false);
+        net_layer<32, 32, false>(l & 1 ? &m_a0 : &m_a1, a.act[l & 1], nullptr, a, sh, sbase, irun);
+    }
+    before_layer([&] { net_stage_weights<32, 16>(a.W[kLayers - 1], a.bias[kLayers - 1], sh, gbase); }, false);
+    net_layer<32, 16, true>(&m_a0, nullptr, a.y, a, sh, sbase, irun);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (warp == kNetMmaWarp)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(sh.tmem), "r"(kNetTmemCols)
                      : "memory");
+    // the last CTA to leave zeroes the counts for the next launch
+    if (tid == 0 && atomicAdd(a.bar + 1, 1u) == gridDim.x - 1) {
+        a.bar[0] = 0u;
+        a.bar[1] = 0u;
+    }
 }
 
 // Framed copy of B images [B][H][Wd][16] (the layer-1 input written
@@ -1812,7 +1819,7 @@ int ensure_net_buffers(s2d_cnn* c) {
               cudaMemset(c->X0f, 0, fp * 16 * sizeof(__nv_bfloat16)) == cudaSuccess &&
               cudaMalloc(&c->F[0], fp * 32 * sizeof(__nv_bfloat16)) == cudaSuccess &&
               cudaMalloc(&c->F[1], fp * 32 * sizeof(__nv_bfloat16)) == cudaSuccess &&
-              cudaMalloc(&c->netbar, 64) == cudaSuccess;
+              cudaMalloc(&c->netbar, 64) == cudaSuccess && cudaMemset(c->netbar, 0, 64) == cudaSuccess;
     if (!ok) {
         cudaFree(c->X0f);
         cudaFree(c->F[0]);
@@ -1855,7 +1862,6 @@ int forward_fused(s2d_cnn* c, int B, bool input_framed) {
     a.stall = c->net_stall ? 1 : 0;
     const long ntiles = (long)((Wd + kNetOutW - 1) / kNetOutW) * ((H + kNetOutH - 1) / kNetOutH) * B;
     const int grid = (int)std::min<long>(ntiles, c->net_grid);
-    C_CUDA(cudaMemsetAsync(c->netbar, 0, sizeof(unsigned int), c->stream));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kNetThreads);
