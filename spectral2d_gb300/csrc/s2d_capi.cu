@@ -211,11 +211,9 @@ struct HostArray {
     bool pageable = false;   // in place through the host page tables
 };
 
-// Whether 16 pages spread over [p, p + n) are resident.  The device writes
-// pageable memory in place only where its pages exist already: a page the
-// GPU touches first is faulted in by the host (45 ms for the 84 MB of fresh
-// np.zeros pages of a 2048^2 output pair on GB300, against 0.4 ms resident),
-// while a staging copy lets the CPU populate them.
+// Whether 16 pages spread over [p, p + n) are resident.  A page that the GPU
+// touches first is faulted in by the host one at a time (45 ms for the 84 MB
+// of fresh np.zeros pages of a 2048^2 output pair, against 0.4 ms resident).
 bool pages_resident(const void* p, size_t n) {
     const long ps = sysconf(_SC_PAGESIZE);
     if (ps <= 0 || n == 0) return false;
@@ -230,23 +228,24 @@ bool pages_resident(const void* p, size_t n) {
     return true;
 }
 
-HostArray host_array(const s2d_handle* h, const double* p) {
+// Makes the pages of [p, p + n) resident and writable in one call, contents
+// kept; false where the kernel cannot.
+bool populate_pages(void* p, size_t n) {
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
+    const long ps = sysconf(_SC_PAGESIZE);
+    if (ps <= 0 || n == 0) return false;
+    const uintptr_t mask = ~(uintptr_t)(ps - 1);
+    const uintptr_t first = (uintptr_t)p & mask, end = ((uintptr_t)p + n + (uintptr_t)ps - 1) & mask;
+    return madvise((void*)first, end - first, MADV_POPULATE_WRITE) == 0;
+}
+
+HostArray host_array(const s2d_handle* h, const double* p, bool write) {
     HostArray a;
     a.host = const_cast<double*>(p);
     if (!p || h->io_copy_only) return a;
-    cudaPointerAttributes at{};
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return a;
-    }
-    if (at.type == cudaMemoryTypeHost) {
-        a.dev = (double*)at.devicePointer;
-    } else if (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged) {
-        if (at.device == h->device) a.dev = a.host;
-    } else if (h->pageable_direct && pages_resident(p, h->ref_bytes)) {
-        a.dev = a.host;
-        a.pageable = true;
-    }
+    a.dev = (double*)device_view(h->device, h->pageable_direct, p, h->ref_bytes, write, &a.pageable);
     return a;
 }
 
@@ -386,6 +385,21 @@ int spectrum_impl(s2d_handle* h, std::vector<double>& Ek) {
 }
 
 }  // namespace
+
+void* s2d::device_view(int device, bool pageable, const void* p, size_t n, bool write, bool* through_tables) {
+    *through_tables = false;
+    void* q = const_cast<void*>(p);
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    if (at.type == cudaMemoryTypeHost) return at.devicePointer;
+    if (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged) return at.device == device ? q : nullptr;
+    if (!pageable || !(pages_resident(p, n) || (write && populate_pages(q, n)))) return nullptr;
+    *through_tables = true;
+    return q;
+}
 
 int s2d::handle_nx(const s2d_handle* h) { return h->cfg.nx; }
 
@@ -759,7 +773,7 @@ S2D_API int s2d_set_state(s2d_handle* h, const double* wC, int32_t cISize, int32
     if (!h || !wC) return fail(S2D_ERR_INVALID, "null argument");
     S2D_TRY(check_ref_dims(h, cISize, nyG));
     S2D_CUDA(cudaSetDevice(h->device));
-    S2D_TRY(upload_ref(h, host_array(h, wC)));
+    S2D_TRY(upload_ref(h, host_array(h, wC, false)));
     S2D_CUDA(cudaStreamSynchronize(h->stream));
     return S2D_OK;
 }
@@ -769,7 +783,7 @@ S2D_API int s2d_get_state(s2d_handle* h, double* wC, double* psiC, int32_t cISiz
     S2D_TRY(check_ref_dims(h, cISize, nyG));
     S2D_CUDA(cudaSetDevice(h->device));
     CopyStreamJoin join{h};
-    const HostArray w = host_array(h, wC), p = host_array(h, psiC);
+    const HostArray w = host_array(h, wC, true), p = host_array(h, psiC, true);
     S2D_TRY(send_zeros(h, w, p));
     return download_ref(h, h->S0, w, p);
 }
@@ -797,7 +811,7 @@ S2D_API int s2d_integrate_one_step_host(s2d_handle* h, double* wC, double* psiC,
     S2D_TRY(check_ref_dims(h, cISize, nyG));
     S2D_CUDA(cudaSetDevice(h->device));
     CopyStreamJoin join{h};
-    const HostArray w = host_array(h, wC), p = host_array(h, psiC);
+    const HostArray w = host_array(h, wC, true), p = host_array(h, psiC, true);
     S2D_TRY(send_zeros(h, w, p));  // only the truncated part: disjoint from the rectangle read in
     S2D_TRY(upload_ref(h, w));
     S2D_TRY(launch_step(h, dt));
@@ -810,7 +824,7 @@ S2D_API int s2d_compute_rhs(s2d_handle* h, double* dW, int32_t cISize, int32_t n
     S2D_CUDA(cudaSetDevice(h->device));
     if (!h->Sdw) S2D_CUDA(cudaMalloc(&h->Sdw, (size_t)h->d.KX * h->d.ldS * h->vsz));
     CopyStreamJoin join{h};
-    const HostArray x = host_array(h, dW);
+    const HostArray x = host_array(h, dW, true);
     S2D_TRY(send_zeros(h, x, HostArray{}));
     S2D_TRY(launch_rhs_stage_any(h, 0, 0.0, nullptr));
     return download_ref(h, h->Sdw, x, HostArray{});

@@ -1351,6 +1351,24 @@ __global__ void k_pack(const float* __restrict__ data, const float* __restrict__
     }
 }
 
+// The same from a caller's (omega, psi) pairs and targets (null: zero).
+__global__ void k_pack_pairs(const float2* __restrict__ in, const float* __restrict__ target, long P, float r0,
+                             float r1, float r2, __nv_bfloat16* x, float* tgt) {
+    for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < P; p += (long)gridDim.x * blockDim.x) {
+        const float2 s = in[p];
+        uint4* xr = reinterpret_cast<uint4*>(x + p * 16);
+        xr[0] = make_uint4(pack_bf16(s.x * r0, s.y * r1), 0u, 0u, 0u);
+        xr[1] = make_uint4(0u, 0u, 0u, 0u);
+        tgt[p] = target ? target[p] * r2 : 0.f;
+    }
+}
+
+// The network's output in physical units.
+__global__ void k_scale_out(const float* __restrict__ y, long P, double scale, float* out) {
+    for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < P; p += (long)gridDim.x * blockDim.x)
+        out[p] = (float)((double)y[p] * scale);
+}
+
 // sum of squares of n doubles, accumulated into *acc (zeroed by the caller)
 template <typename T>
 __global__ void k_sumsq(const T* __restrict__ v, long n, double* acc) {
@@ -1760,6 +1778,8 @@ struct s2d_cnn {
     __nv_bfloat16* dZk[kLayers - 1] = {};
     bool keep = false;
     float *Y = nullptr, *tgt = nullptr;
+    float* stage = nullptr;      // a caller's batch that the device cannot read in place
+    bool pageable_direct = false;   // the device reads ordinary host memory in place
     float* part = nullptr;
     long part_n = 0;
     int wg_blocks = 0;
@@ -1998,34 +2018,40 @@ uint64_t mix64(uint64_t x) {
     return x ^ (x >> 31);
 }
 
+// The network input (and the normalised target) of a batch from the caller's
+// arrays, read in place where the device reaches them, else through a staging
+// buffer kept with the network.  Asynchronous on the network's stream: the
+// caller waits for it before it returns.
 int upload_host_batch(s2d_cnn* c, const float* x, const float* target, int B) {
-    // host (omega, psi) pairs -> temporary dataset slots at the end of a
-    // private staging area, then the packing kernel
-    const long HW = (long)c->H * c->Wd;
-    std::vector<float> s((size_t)B * HW * 3);
-    for (long i = 0; i < (long)B * HW; ++i) {
-        s[3 * i] = x[2 * i];
-        s[3 * i + 1] = x[2 * i + 1];
-        s[3 * i + 2] = target ? target[i] : 0.f;
+    const long P = (long)B * c->H * c->Wd;
+    bool tables;
+    const float* xd = (const float*)device_view(c->device, c->pageable_direct, x, 2 * P * sizeof(float), false, &tables);
+    const float* td = target ? (const float*)device_view(c->device, c->pageable_direct, target, P * sizeof(float),
+                                                         false, &tables)
+                             : nullptr;
+    if ((!xd || (target && !td)) && !c->stage)
+        C_CUDA(cudaMalloc(&c->stage, 3 * (size_t)c->maxB * c->H * c->Wd * sizeof(float)));
+    if (!xd) {
+        C_CUDA(cudaMemcpyAsync(c->stage, x, 2 * P * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+        xd = c->stage;
     }
-    float* tmp = nullptr;
-    int* idx = nullptr;
-    C_CUDA(cudaMalloc(&tmp, s.size() * sizeof(float)));
-    C_CUDA(cudaMalloc(&idx, sizeof(int) * B));
-    std::vector<int> id(B);
-    for (int b = 0; b < B; ++b) id[b] = b;
-    C_CUDA(cudaMemcpyAsync(tmp, s.data(), s.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    C_CUDA(cudaMemcpyAsync(idx, id.data(), sizeof(int) * B, cudaMemcpyHostToDevice, c->stream));
-    k_pack<<<nblocks((long)B * HW, 256), 256, 0, c->stream>>>(tmp, nullptr, idx, B, HW, (float)(1.0 / c->scale[0]),
-                                                              (float)(1.0 / c->scale[1]), (float)(1.0 / c->scale[2]),
-                                                              c->X0, c->tgt);
-    cudaError_t e = cudaGetLastError();
-    cudaStreamSynchronize(c->stream);
-    cudaFree(tmp);
-    cudaFree(idx);
-    if (e != cudaSuccess) return cerr(S2D_ERR_CUDA, cudaGetErrorString(e));
+    if (target && !td) {
+        C_CUDA(cudaMemcpyAsync(c->stage + 2 * P, target, P * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+        td = c->stage + 2 * P;
+    }
+    k_pack_pairs<<<nblocks(P, 256), 256, 0, c->stream>>>((const float2*)xd, td, P, (float)(1.0 / c->scale[0]),
+                                                         (float)(1.0 / c->scale[1]), (float)(1.0 / c->scale[2]), c->X0,
+                                                         c->tgt);
+    C_CUDA(cudaGetLastError());
     return S2D_OK;
 }
+
+// Waits for the network's stream on every exit of a host-array call, so that
+// nothing reads or writes the caller's arrays once it has returned.
+struct NetStreamJoin {
+    s2d_cnn* c;
+    ~NetStreamJoin() { cudaStreamSynchronize(c->stream); }
+};
 
 // Physical w (and psi) of a spectral field of the handle on its collocation grid.
 template <typename T>
@@ -2231,6 +2257,12 @@ S2D_API int s2d_cnn_create(int32_t grid, int32_t max_batch, uint64_t seed, int32
     c->device = device;
     c->H = c->Wd = grid;
     c->maxB = max_batch;
+    {
+        const char* io = std::getenv("S2D_HOST_IO");
+        int pageable = 0;
+        if (cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, device) != cudaSuccess) pageable = 0;
+        c->pageable_direct = pageable == 1 && !(io && std::strcmp(io, "copy") == 0);
+    }
     // S2D_CNN_LAYERWISE=1: gradient-free forward passes one launch per layer
     // (for comparisons; s2d_cnn_set_fused switches it per network)
     if (const char* e = std::getenv("S2D_CNN_LAYERWISE")) c->fused = e[0] == '\0' || e[0] == '0';
@@ -2334,7 +2366,8 @@ S2D_API void s2d_cnn_destroy(s2d_cnn* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     void* ptrs[] = {c->master, c->grad, c->m, c->v, c->X0, c->dZ6, c->dZa, c->dZb, c->Y, c->tgt, c->part,
-                    c->lpart, c->idx, c->data, c->amp, c->sumsq, c->cflags, c->X0f, c->F[0], c->F[1], c->netbar};
+                    c->lpart, c->idx, c->data, c->amp, c->sumsq, c->cflags, c->X0f, c->F[0], c->F[1], c->netbar,
+                    c->stage};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     for (int l = 0; l < kLayers; ++l) {
@@ -2405,15 +2438,19 @@ S2D_API int s2d_cnn_get_band(const s2d_cnn* c, double* k_min) {
 S2D_API int s2d_cnn_forward_host(s2d_cnn* c, const float* x, int32_t B, float* y) {
     if (!c || !x || !y || B < 1 || B > c->maxB) return cerr(S2D_ERR_INVALID, "bad batch");
     C_CUDA(cudaSetDevice(c->device));
+    NetStreamJoin join{c};
     int r = upload_host_batch(c, x, nullptr, B);
     if (r != S2D_OK) return r;
     r = forward(c, B, false);
     if (r != S2D_OK) return r;
     const long P = (long)B * c->H * c->Wd;
-    std::vector<float> out(P);
-    C_CUDA(cudaMemcpyAsync(out.data(), c->Y, P * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+    bool tables;
+    float* yd = (float*)device_view(c->device, c->pageable_direct, y, P * sizeof(float), true, &tables);
+    float* dst = yd ? yd : c->tgt;   // the targets are unused here
+    k_scale_out<<<nblocks(P, 256), 256, 0, c->stream>>>(c->Y, P, c->scale[2], dst);
+    C_CUDA(cudaGetLastError());
+    if (!yd) C_CUDA(cudaMemcpyAsync(y, dst, P * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
     C_CUDA(cudaStreamSynchronize(c->stream));
-    for (long i = 0; i < P; ++i) y[i] = (float)(out[i] * c->scale[2]);
     return s2d_cnn_status(c);
 }
 
@@ -2421,6 +2458,7 @@ S2D_API int s2d_cnn_grad_host(s2d_cnn* c, const float* x, const float* target, i
                               double* loss) {
     if (!c || !x || !target || B < 1 || B > c->maxB) return cerr(S2D_ERR_INVALID, "bad batch");
     C_CUDA(cudaSetDevice(c->device));
+    NetStreamJoin join{c};
     int r = upload_host_batch(c, x, target, B);
     if (r != S2D_OK) return r;
     if ((r = forward(c, B, true)) != S2D_OK) return r;

@@ -330,6 +330,12 @@ namespace s2d {
 // s2d_create with an optional external stream (not owned by the handle).
 int create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handle** out);
 
+// The address at which the device reaches n bytes of a caller's array in
+// place: page-locked or device memory, or (pageable) ordinary host memory
+// through the host page tables where its pages are resident; writable arrays
+// whose pages are not are populated first.  Null: copy instead.
+void* device_view(int device, bool pageable, const void* p, size_t n, bool write, bool* through_tables);
+
 // Shared-memory attribute setup (called once per process and device).
 cudaError_t configure_kernels(int max_smem_optin);
 

@@ -120,7 +120,7 @@ class Spectral2D:
 
     # -- state ----------------------------------------------------------------
     def _new(self) -> np.ndarray:
-        return np.zeros(self.shape, dtype=np.complex128)
+        return np.empty(self.shape, dtype=np.complex128)   # the library writes every element
 
     def set_state(self, wC: np.ndarray) -> None:
         w = np.ascontiguousarray(wC, dtype=np.complex128)
@@ -427,7 +427,7 @@ class ClosureNet:
     def forward(self, x: np.ndarray) -> np.ndarray:
         """x: (B, grid, grid, 2) (w, psi) -> (B, grid, grid) Pi."""
         x = np.ascontiguousarray(x, dtype=np.float32)
-        y = np.zeros(x.shape[:3], dtype=np.float32)
+        y = np.empty(x.shape[:3], dtype=np.float32)
         L.check(self._L.s2d_cnn_forward_host(self._c, _fptr(x), x.shape[0], _fptr(y)))
         return y
 
