@@ -276,17 +276,23 @@ int upload_ref(s2d_handle* h, const HostArray& w) {
 // Outputs in the reference layout are zero outside the retained rectangle
 // (Truncate, src/Spectral.F90:788-802): columns kx > K of rows 0..K and
 // M-K..M-1, and the whole rows K+1..M-K-1.  That part does not depend on the
-// state, so it is written on the handle's second stream, which a host-array
-// step issues before the step and so overlaps with it: by a small kernel for
-// pageable arrays reached in place (a copy into pageable memory may hold the
-// host until it ends), else by copies from a device buffer of zeros.
-int send_zeros(s2d_handle* h, const HostArray& a, const HostArray& b) {
+// state, so it is written on the handle's second stream, concurrently with
+// the step: by a small kernel for pageable arrays reached in place (a copy
+// into pageable memory may hold the host until it ends), else by copies from
+// a device buffer of zeros.  Called twice: the kernel goes out before the
+// upload (later it would take SMs from the step: 2048^2 FP32 1.62 against
+// 1.50 ms), the copies after the step's launches, which would wait for the
+// host to issue them (1.35 against 1.31 ms).
+int send_zeros(s2d_handle* h, const HostArray& a, const HostArray& b, bool before) {
     if (!a.host && !b.host) return S2D_OK;
     const int K = h->d.K, M = h->d.M, C = h->grid.cISize;
     if (!h->xstream) S2D_CUDA(cudaStreamCreateWithFlags(&h->xstream, cudaStreamNonBlocking));
-    if (a.pageable || b.pageable)
-        S2D_CUDA(launch_zero_truncated(h->d, C, a.pageable ? a.dev : nullptr, b.pageable ? b.dev : nullptr, 48,
-                                       h->xstream));
+    if (before) {
+        if (a.pageable || b.pageable)
+            S2D_CUDA(launch_zero_truncated(h->d, C, a.pageable ? a.dev : nullptr, b.pageable ? b.dev : nullptr, 48,
+                                           h->xstream));
+        return S2D_OK;
+    }
     const size_t pitch = (size_t)C * 2 * sizeof(double);
     const size_t kx_off = (size_t)h->d.KX * 2 * sizeof(double);
     const size_t tail = pitch - kx_off;                       // columns K+1..C-1 of one row
@@ -784,7 +790,8 @@ S2D_API int s2d_get_state(s2d_handle* h, double* wC, double* psiC, int32_t cISiz
     S2D_CUDA(cudaSetDevice(h->device));
     CopyStreamJoin join{h};
     const HostArray w = host_array(h, wC, true), p = host_array(h, psiC, true);
-    S2D_TRY(send_zeros(h, w, p));
+    S2D_TRY(send_zeros(h, w, p, true));
+    S2D_TRY(send_zeros(h, w, p, false));
     return download_ref(h, h->S0, w, p);
 }
 
@@ -812,9 +819,10 @@ S2D_API int s2d_integrate_one_step_host(s2d_handle* h, double* wC, double* psiC,
     S2D_CUDA(cudaSetDevice(h->device));
     CopyStreamJoin join{h};
     const HostArray w = host_array(h, wC, true), p = host_array(h, psiC, true);
-    S2D_TRY(send_zeros(h, w, p));  // only the truncated part: disjoint from the rectangle read in
+    S2D_TRY(send_zeros(h, w, p, true));  // only the truncated part: disjoint from the rectangle read in
     S2D_TRY(upload_ref(h, w));
     S2D_TRY(launch_step(h, dt));
+    S2D_TRY(send_zeros(h, w, p, false));
     return download_ref(h, h->S0, w, p);
 }
 
@@ -825,8 +833,9 @@ S2D_API int s2d_compute_rhs(s2d_handle* h, double* dW, int32_t cISize, int32_t n
     if (!h->Sdw) S2D_CUDA(cudaMalloc(&h->Sdw, (size_t)h->d.KX * h->d.ldS * h->vsz));
     CopyStreamJoin join{h};
     const HostArray x = host_array(h, dW, true);
-    S2D_TRY(send_zeros(h, x, HostArray{}));
+    S2D_TRY(send_zeros(h, x, HostArray{}, true));
     S2D_TRY(launch_rhs_stage_any(h, 0, 0.0, nullptr));
+    S2D_TRY(send_zeros(h, x, HostArray{}, false));
     return download_ref(h, h->Sdw, x, HostArray{});
 }
 
