@@ -225,8 +225,7 @@ __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double
         fx_bf4<true>(z[b]);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            const int a = (int)(z[b][r].x >> 32), c = (int)(z[b][r].y >> 32);
-            m2 = max(m2, max(a ^ (a >> 31), c ^ (c >> 31)));
+            m2 = max(m2, max(abs((int)(z[b][r].x >> 32)), abs((int)(z[b][r].y >> 32))));
         }
     }
     fx_reduce_max(&words[2], m2, lane, whole);

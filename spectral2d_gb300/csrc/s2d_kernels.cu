@@ -46,9 +46,9 @@ namespace s2d {
 // time -- measured slower at 2048^2: 0.81 / 0.82 against 0.774 ms per step.)
 // ------------------------------------------------------------------------
 template <int B>
-constexpr int kMaxThreads = B == 1 ? 256 : 512;
+constexpr int kMaxThreads = B == 1 ? 256 : (B == 3 ? 384 : 512);
 template <typename T, int B>
-constexpr int kMinBlocks = B == 1 ? (sizeof(T) == 8 ? 3 : 4) : (B == 2 ? 2 : 1);
+constexpr int kMinBlocks = B == 1 ? (sizeof(T) == 8 ? 3 : 4) : (B >= 2 ? 2 : 1);
 template <typename T>
 int budget(int threads) {
     return threads <= 256 ? 1 : (sizeof(T) == 4 ? 2 : 0);
@@ -125,7 +125,10 @@ __global__ void __launch_bounds__(256) k_stage(Dims d, const typename Vec<T>::t*
 
 // ---- FP64, direct plans (s2d_fxstep.cuh) ---------------------------------
 // E elements per thread: 12, or 4 for small grids.  CTAs of at most 256
-// threads: three per SM (80 registers); up to 512: one.
+// threads: three per SM (B = 1, 80 registers); up to 384: two (B = 3, 80; one
+// at 128 took 5.77 against 5.50 ms of the 3072^2 step); up to 512: K1 two
+// (B = 2, 64), whose loads and stores gain more than its spills cost (4096^2
+// 2.37 -> 2.31 ms), K2 and K3 one (B = 0, 128; two: 4.5 -> 5.0, 2.8 -> 3.3 ms).
 template <int E, int B>
 __global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<double, B>))
     k_fx_yinv(Dims d, const double2* __restrict__ S, const double* __restrict__ rk2, FieldSet fs,
@@ -717,11 +720,11 @@ cudaError_t Kern<T>::yinv(const Dims& d, const void* S, const double* rk2, const
     if constexpr (sizeof(T) == 8) {
         const FxTw* ft = (const FxTw*)tw;
         if (!d.direct) return launch_k(k_yinv<T, 0>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
-        if (d.Tg * 4 == d.M)
-            return L.threads <= 256 ? launch_k(k_fx_yinv<4, 1>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G)
-                                    : launch_k(k_fx_yinv<4, 0>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G);
-        return L.threads <= 256 ? launch_k(k_fx_yinv<12, 1>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G)
-                                : launch_k(k_fx_yinv<12, 0>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G);
+        const bool four = d.Tg * 4 == d.M;
+        return launch_k(L.threads <= 256   ? (four ? k_fx_yinv<4, 1> : k_fx_yinv<12, 1>)
+                        : L.threads <= 384 ? (four ? k_fx_yinv<4, 0> : k_fx_yinv<12, 3>)
+                                           : (four ? k_fx_yinv<4, 0> : k_fx_yinv<12, 2>),
+                        nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, ft, L.G);
     } else {
         if (!d.direct) return launch_k(k_yinv<T, 2>, nb, L.threads, L.smem, st, L.pdl, d, s, rk2, fs, t, L.G);
         const bool four = d.Tg * 4 == d.M;
@@ -756,11 +759,11 @@ cudaError_t Kern<T>::xpass_bas(const Dims& d, void* Iu, void* Iv, const void* tw
     if constexpr (sizeof(T) == 8) {
         const FxTw* ft = (const FxTw*)tw;
         if (!d.direct) return launch_k(k_xpass_bas<T, 0>, nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
-        if (d.Tg * 4 == d.M)
-            return L.threads <= 256 ? launch_k(k_fx_xpass<4, 1>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale)
-                                    : launch_k(k_fx_xpass<4, 0>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale);
-        return L.threads <= 256 ? launch_k(k_fx_xpass<12, 1>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale)
-                                : launch_k(k_fx_xpass<12, 0>, nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale);
+        const bool four = d.Tg * 4 == d.M;
+        return launch_k(L.threads <= 256   ? (four ? k_fx_xpass<4, 1> : k_fx_xpass<12, 1>)
+                        : L.threads <= 384 ? (four ? k_fx_xpass<4, 0> : k_fx_xpass<12, 3>)
+                                           : (four ? k_fx_xpass<4, 0> : k_fx_xpass<12, 0>),
+                        nb, L.threads, L.smem, st, L.pdl, d, u, v, ft, L.G, scale);
     } else {
         if (!d.direct) return launch_k(k_xpass_bas<T, 2>, nb, L.threads, L.smem, st, L.pdl, d, u, v, t, L.G, scale);
         const bool four = d.Tg * 4 == d.M;
@@ -805,10 +808,10 @@ cudaError_t Kern<T>::yfwd_col(const Dims& d, const void* Iu, const void* Iv, voi
     if constexpr (sizeof(T) == 8) {   // FP64 runs alone split their K3
         const FxTw* ft = (const FxTw*)tw;
         if (d.direct)
-            return L.threads <= 256 ? launch_k(k_fx_yfwd_col<12, 1>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v,
-                                               (VT*)Fu, (VT*)Fv, ft, L.G)
-                                    : launch_k(k_fx_yfwd_col<12, 0>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v,
-                                               (VT*)Fu, (VT*)Fv, ft, L.G);
+            return launch_k(L.threads <= 256   ? k_fx_yfwd_col<12, 1>
+                            : L.threads <= 384 ? k_fx_yfwd_col<12, 3>
+                                               : k_fx_yfwd_col<12, 0>,
+                            2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v, (VT*)Fu, (VT*)Fv, ft, L.G);
         return launch_k(k_yfwd_col<T>, 2 * ncg, L.threads, L.smem, st, L.pdl, d, u, v, (VT*)Fu, (VT*)Fv,
                         (const VT*)tw, L.G);
     }
@@ -976,15 +979,18 @@ cudaError_t configure_kernels(int max_smem_optin) {
     S2D_SET((k_f32_yfwd_rk3<4, 1>));
     S2D_SET((k_f32_yfwd_rk3<4, 2>));
     S2D_SET((k_fx_yinv<12, 1>));
-    S2D_SET((k_fx_yinv<12, 0>));
+    S2D_SET((k_fx_yinv<12, 2>));
+    S2D_SET((k_fx_yinv<12, 3>));
     S2D_SET((k_fx_yinv<4, 1>));
     S2D_SET((k_fx_yinv<4, 0>));
     S2D_SET((k_fx_xpass<12, 1>));
     S2D_SET((k_fx_xpass<12, 0>));
+    S2D_SET((k_fx_xpass<12, 3>));
     S2D_SET((k_fx_xpass<4, 1>));
     S2D_SET((k_fx_xpass<4, 0>));
     S2D_SET((k_fx_yfwd_col<12, 1>));
     S2D_SET((k_fx_yfwd_col<12, 0>));
+    S2D_SET((k_fx_yfwd_col<12, 3>));
     S2D_SET(k_fx_yfwd_rk3<12>);
     S2D_SET(k_fx_yfwd_rk3<4>);
     S2D_SET((k_yinv<double, 0>));
