@@ -154,7 +154,11 @@ int launch_rhs_stage(s2d_handle* h, int stage, double dt, cudaEvent_t* ev, cudaE
     S2D_CUDA(Kern<T>::yinv(d, win, bas ? h->rk2s : h->rk2, fs, h->tw, h->stream, small ? h->S_yinv : h->L_yinv));
     if (ev) S2D_CUDA(cudaEventRecord(ev[1], h->stream));
     if (bas) S2D_CUDA(Kern<T>::xpass_bas(d, h->I[0], h->I[1], h->tw, h->stream, small ? h->S_xrow : h->L_xrow, true));
-    else S2D_CUDA(Kern<T>::xpass_rhs(h->d, h->I[0], h->I[1], h->I[2], h->tw, h->stream, h->L_xpass));
+    else {
+        Dims dx = h->d;
+        if (h->xp_four) dx.Tg = dx.M / 4;
+        S2D_CUDA(Kern<T>::xpass_rhs(dx, h->I[0], h->I[1], h->I[2], h->tw, h->stream, h->L_xpass, h->xp_three));
+    }
     if (ev) S2D_CUDA(cudaEventRecord(ev[2], h->stream));
     if (h->Fv && !small) {
         // K3 in two launches (FP64, Basdevant): the column FFTs take three
@@ -631,7 +635,18 @@ int s2d::create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handl
     const int nf = h->ph.form == S2D_NL_BASDEVANT ? 2 : 3;
     if ((rr = pick_launch(h, d.Tg, tb, tgt, (long)nf * d.KX, &h->L_yinv, "inverse y-pass")) != S2D_OK)
         return bail(rr);
-    if ((rr = pick_launch(h, d.Tg, 2 * tb, tgt, d.M / 2, &h->L_xpass, "x-pass")) != S2D_OK) return bail(rr);
+    // Conservative x-pass: three groups per row pair while the grid has few
+    // pairs (k_xpass_rhs3), with 4 elements per thread on the smallest.  us per
+    // step, one group of 12 / three of 12 / three of 4:
+    //   FP64  64^2 203 / 115 / 72, 256^2 227 / 133 / 127, 384^2 271 / 182 / 190,
+    //         512^2 299 / 289, 576^2 387 / 338, 768^2 493 / 632
+    //   FP32  64^2 78 / 47 / 39, 256^2 108 / 67 / 53, 384^2 106 / 80 / 74,
+    //         512^2 125 / 100, 576^2 176 / 145, 864^2 320 / 320
+    h->xp_three = d.M <= 864;
+    h->xp_four = d.M <= (h->prec == S2D_FP64 ? 384 : 576);
+    if ((rr = pick_launch(h, h->xp_three ? 3 * (h->xp_four ? d.M / 4 : d.Tg) : d.Tg, (h->xp_three ? 3 : 2) * tb, tgt,
+                          d.M / 2, &h->L_xpass, "x-pass")) != S2D_OK)
+        return bail(rr);
     // forward y-pass: G columns x 2 fields, run in rounds of c transforms
     auto pick_yfwd = [&](int Tg, Launch* out_l) {
         Launch L{};

@@ -508,18 +508,19 @@ __device__ __forceinline__ void fx_middle(longlong2* buf, const Dims& d, int lan
 }
 
 // ---- the general FP64 transform, FP64 in and out (fft_run) -----------------
-// First pass: the 12 elements of the thread from FP64, their common exponent
+// First pass: the E elements of the thread from FP64, their common exponent
 // emax, the sum of magnitudes, a radix-R DFT without twiddles.  PRUNE: radix 3
 // with the middle input zero but for j = 0 (see fft_pass3_midzero).
-template <int R, bool INV, bool PRUNE>
+template <int E, int R, bool INV, bool PRUNE>
 __device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg, int n0, int* words) {
-    constexpr int NB = kElemsPerThread / R;
+    constexpr int NB = kFxNB<E, R>;
     double2 z[NB][R];
     const int stride = M / R;
     int mx = 0;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
+        if (!fx_on<E, R>(j, M)) continue;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if (PRUNE && r == 1 && (b > 0 || j > 0)) continue;
@@ -535,6 +536,7 @@ __device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg,
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
+        if (!fx_on<E, R>(j, M)) continue;
         fx2 v[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -558,9 +560,8 @@ __device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg,
 
 // The FP64 transform (see fft_run).  A transform with an infinity or NaN
 // gives NaN throughout.
-template <bool INV>
+template <bool INV, int E>
 __device__ __forceinline__ void fx_run(longlong2* buf, const Dims& d, int lane, const FxTw* __restrict__ tab) {
-    constexpr int E = kElemsPerThread;
     int* words = fx_words() + ((int)threadIdx.x - lane);
     if (lane == 0) {
         words[0] = 0;
@@ -570,10 +571,10 @@ __device__ __forceinline__ void fx_run(longlong2* buf, const Dims& d, int lane, 
     const int R0 = d.radix[0];
     const int n0 = R0 == 4 ? 4 : 3;
     int emax;
-    if (INV && R0 == 3 && 3 * d.K == d.M) emax = fx_first<3, INV, INV>(buf, d.M, lane, d.Tg, n0, words);
-    else if (R0 == 3) emax = fx_first<3, INV, false>(buf, d.M, lane, d.Tg, n0, words);
-    else if (R0 == 4) emax = fx_first<4, INV, false>(buf, d.M, lane, d.Tg, n0, words);
-    else emax = fx_first<2, INV, false>(buf, d.M, lane, d.Tg, n0, words);
+    if (INV && R0 == 3 && 3 * d.K == d.M) emax = fx_first<E, 3, INV, INV>(buf, d.M, lane, d.Tg, n0, words);
+    else if (R0 == 3) emax = fx_first<E, 3, INV, false>(buf, d.M, lane, d.Tg, n0, words);
+    else if (R0 == 4) emax = fx_first<E, 4, INV, false>(buf, d.M, lane, d.Tg, n0, words);
+    else emax = fx_first<E, 2, INV, false>(buf, d.M, lane, d.Tg, n0, words);
     const unsigned sum = (unsigned)words[512];
     const float per = fx_per(n0);
     int Ns = R0, t = 0;
@@ -631,15 +632,15 @@ __device__ __forceinline__ void f32_passes(float2* buf, const Dims& d, int lane,
 // that callers may fill buf just before.  tw points at the handle's twiddles
 // (Dims::twoff, tab_bytes).  Inverse transforms of truncated spectra (input
 // zero for K < n < M - K, K = M/3: the inverse transforms of this library)
-// take the pruned first radix-3 pass.
-template <bool INV, typename VT>
+// take the pruned first radix-3 pass.  E elements per thread (d.Tg = M / E).
+template <bool INV, int E = kElemsPerThread, typename VT>
 __device__ __forceinline__ void fft_run(VT* buf, const Dims& d, int lane, const VT* __restrict__ tw) {
     using T = decltype(buf[0].x);
     if constexpr (sizeof(T) == 8) {
-        fx_run<INV>(reinterpret_cast<longlong2*>(buf), d, lane, reinterpret_cast<const FxTw*>(tw));
+        fx_run<INV, E>(reinterpret_cast<longlong2*>(buf), d, lane, reinterpret_cast<const FxTw*>(tw));
     } else {
         __syncthreads();
-        f32_passes<kElemsPerThread, INV>(buf, d, lane, tw, 0, d.npass);
+        f32_passes<E, INV>(buf, d, lane, tw, 0, d.npass);
     }
 }
 

@@ -192,7 +192,7 @@ struct Kern {
     static cudaError_t yinv(const Dims& d, const void* S, const double* rk2, const FieldSet& fs,
                             const void* tw, cudaStream_t st, const Launch& L);
     static cudaError_t xpass_rhs(const Dims& d, void* Iu, void* Iv, const void* Iw, const void* tw,
-                                 cudaStream_t st, const Launch& L);
+                                 cudaStream_t st, const Launch& L, bool three);
     // prescaled: u and v came from the rk2s table (scaled by sqrt(0.5)/M), so
     // their products carry the 1/(2 M^2) of the forward transform already
     static cudaError_t xpass_bas(const Dims& d, void* Iu, void* Iv, const void* tw, cudaStream_t st,
@@ -316,6 +316,7 @@ struct s2d_handle {
     // per thread (Dims::Tg = M / 4), K3 in one launch
     bool small = false;
     s2d::Launch S_yinv, S_xrow, S_yfwd, S_ystore;
+    bool xp_three = false, xp_four = false;   // conservative x-pass: three groups per row pair; 4 elements per thread
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     double graph_dt = 0.0;

@@ -244,6 +244,43 @@ __global__ void __launch_bounds__(512) k_xpass_rhs(Dims d, typename Vec<T>::t* I
     }
 }
 
+// The same on three groups per row pair: the inverse FFTs of omega, of row y1
+// and of row y2 run side by side, then the forward ones of the two rows (the
+// omega group transforms along with them for the barriers).  A small grid has
+// fewer row pairs than the SMs take, and the kernel's time is that of its chain
+// of transforms: two here, five in k_xpass_rhs.  E elements per thread
+// (d.Tg = M / E).  Every value takes the same operations as there.
+template <typename T, int E>
+__global__ void __launch_bounds__(512) k_xpass_rhs3(Dims d, typename Vec<T>::t* Iu, typename Vec<T>::t* Iv,
+                                                    const typename Vec<T>::t* __restrict__ Iw,
+                                                    const typename Vec<T>::t* __restrict__ tw, int G, T scale) {
+    using VT = typename Vec<T>::t;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_enter();
+    const int g = threadIdx.x / d.Tg;
+    const int lane = threadIdx.x - g * d.Tg;
+    const int pg = g / 3, role = g - 3 * pg;   // role 0: omega, 1: row y1, 2: row y2
+    const int p = blockIdx.x * G + pg;
+    const bool active = p < d.M / 2;
+    const int y1 = active ? 2 * p : 0;
+    VT* Z = reinterpret_cast<VT*>(smem_raw) + (size_t)g * d.M;
+    const VT* W = Z - (size_t)role * d.M;
+    VT* urow = Iu + (size_t)(y1 + (role == 2)) * d.ldI;
+    VT* vrow = Iv + (size_t)(y1 + (role == 2)) * d.ldI;
+    build_pair<E>(Z, role ? urow : Iw + (size_t)y1 * d.ldI, role ? vrow : Iw + (size_t)(y1 + 1) * d.ldI, d, lane,
+                  active);
+    fft_run<true, E>(Z, d, lane, tw);
+    if (role) {
+        for (int n = lane; n < d.M; n += d.Tg) {
+            const VT z = Z[n];
+            const T s = role == 2 ? W[n].y : W[n].x;
+            Z[n] = mk<VT>(z.x * s, z.y * s);
+        }
+    }
+    fft_run<false, E>(Z, d, lane, tw);
+    extract_pair(Z, urow, vrow, d, lane, active && role, scale);
+}
+
 // ------------------------------------------------------------------------
 // Layout conversion between the reference's (cISize, nyG) complex128 array
 // and the compact state.
@@ -736,10 +773,13 @@ cudaError_t Kern<T>::yinv(const Dims& d, const void* S, const double* rk2, const
 
 template <typename T>
 cudaError_t Kern<T>::xpass_rhs(const Dims& d, void* Iu, void* Iv, const void* Iw, const void* tw,
-                               cudaStream_t st, const Launch& L) {
+                               cudaStream_t st, const Launch& L, bool three) {
     using VT = typename Vec<T>::t;
     const int pairs = d.M / 2;
     const T scale = (T)(0.5 / ((double)d.M * (double)d.M));
+    if (three)
+        return launch_k(d.Tg * 4 == d.M ? k_xpass_rhs3<T, 4> : k_xpass_rhs3<T, 12>, (pairs + L.G - 1) / L.G, L.threads,
+                        L.smem, st, L.pdl, d, (VT*)Iu, (VT*)Iv, (const VT*)Iw, (const VT*)tw, L.G, scale);
     return launch_k(k_xpass_rhs<T>, (pairs + L.G - 1) / L.G, L.threads, L.smem, st, L.pdl, d, (VT*)Iu, (VT*)Iv,
                     (const VT*)Iw, (const VT*)tw, L.G, scale);
 }
@@ -997,6 +1037,10 @@ cudaError_t configure_kernels(int max_smem_optin) {
     S2D_SET((k_yinv<float, 2>));
     S2D_SET(k_xpass_rhs<double>);
     S2D_SET(k_xpass_rhs<float>);
+    S2D_SET((k_xpass_rhs3<double, 4>));
+    S2D_SET((k_xpass_rhs3<double, 12>));
+    S2D_SET((k_xpass_rhs3<float, 4>));
+    S2D_SET((k_xpass_rhs3<float, 12>));
     S2D_SET((k_xpass_bas<double, 0>));
     S2D_SET((k_xpass_bas<float, 2>));
     S2D_SET(k_yfwd_col<double>);

@@ -150,14 +150,13 @@ __device__ __forceinline__ void yinv_body(const Dims& d, const typename Vec<T>::
 // Hermitian extension of two half-spectrum rows X, Y (kx in [0,K]) packed as
 // Z = X + iY over the full length M; the kx=0 entries contribute their real
 // parts only (the c2r convention of FFTW, used by src/Spectral.F90:780).
-template <typename VT>
+template <int E = kElemsPerThread, typename VT>
 __device__ __forceinline__ void build_pair(VT* buf, const VT* __restrict__ X, const VT* __restrict__ Y,
                                            const Dims& d, int lane, bool active) {
     using T = decltype(buf[0].x);
-    // M = kElemsPerThread * Tg; all loads in flight for FP32 (FP64 K2 would
-    // spill at its 80-register budget)
-#pragma unroll(sizeof(T) == 8 ? 1 : kElemsPerThread)
-    for (int i = 0; i < kElemsPerThread; ++i) {
+    // M = E * Tg; all loads in flight for FP32 (FP64 would spill)
+#pragma unroll(sizeof(T) == 8 ? 1 : E)
+    for (int i = 0; i < E; ++i) {
         const int n = lane + i * d.Tg;
         VT z = mk<VT>((T)0, (T)0);
         if (active) {

@@ -134,3 +134,21 @@ def test_four_and_twelve_elements_per_thread_give_the_same_bits(mods, n):
         s.set_state(w)
         s.integrate_steps(2, 1e-3)
         assert np.array_equal(ens.runs[0].get_state()[0], s.get_state()[0])
+
+
+# the conservative x-pass: three groups of 4 elements per thread up to n = 256
+# (FP64) or 384 (FP32), three of 12 up to 576, one group above; the orders of
+# the radices at each
+@pytest.mark.parametrize("plan", [0, 1, 2])
+@pytest.mark.parametrize("precision, tol", [("fp64", 1e-13), ("fp32", 5e-6)])
+@pytest.mark.parametrize("n", [8, 24, 256, 288, 384, 432, 576, 648])
+def test_conservative_rhs_at_the_sizes_where_its_kernel_changes(mods, n, precision, tol, plan):
+    _, S2D = mods
+    g = O.get_grid_size(n, n)
+    w = O.truncate(O.random_state(g, 7 + n, decay=0.02), g)
+    with S2D(n, nu=0.01, nonlinear_form="conservative", precision=precision) as s:
+        s.fft_plan = plan
+        s.set_state(w)
+        dW = s.compute_rhs()
+    ref, _ = O.compute_rhs(w, O.truncate(O.compute_psi(w, g), g), g, 0.01, round_trip=False)
+    assert O.rel_l2(dW, O.truncate(ref, g)) < tol
