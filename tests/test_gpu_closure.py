@@ -465,3 +465,27 @@ def test_trained_closure_meets_the_spectrum_bar_on_a_held_out_seed(S):
           f"none mean {m0:.4f} max {x0:.3f}")
     assert mc < 0.10
     assert mc < 0.5 * m0
+
+
+@pytest.mark.parametrize("scale", [20.0, 300.0, 1e20])
+def test_pre_activations_far_from_zero_vs_oracle(S, scale):
+    """The activation takes its paired form below |z| = 12.5 and the scalar one
+    for groups that hold a larger value: inputs whose first layer straddles
+    that bound, lies mostly beyond it, and overflows exp.  BF16 results of an
+    FP32 sum: within 1e-3 of the oracle's on the same values, as per layer
+    above."""
+    grid, B = 24, 2
+    rng = np.random.default_rng(11)
+    with S.ClosureNet(grid, max_batch=2, seed=3) as net:
+        net.set_scales([1.0, 1.0, 1.0])
+        net.keep_layer_grads(True)
+        p = net.get_params()
+        x = (scale * rng.standard_normal((B, grid, grid, 2))).astype(np.float32)
+        net.grad(x, np.zeros((B, grid, grid), np.float32))
+        A = [net.tensor(0, l, B).astype(np.float64) for l in range(2)]
+        Z = net.tensor(1, 0, B).astype(np.float64)
+    (W, b), ci, co = _oracle_params(p)[0], CO.CHANNELS[0], CO.CHANNELS[1]
+    z = CO.conv(A[0][..., :ci], W, b)
+    assert np.abs(z).max() > 12.5
+    assert _rel(Z[..., :co], _bf(z)) < 1e-3
+    assert _rel(A[1][..., :co], _bf(CO.gelu(z))) < 1e-3
