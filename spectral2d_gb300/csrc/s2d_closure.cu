@@ -1145,12 +1145,19 @@ __global__ void __launch_bounds__(256) k_conv_wgrad(const __nv_bfloat16* __restr
 //     row block dy (32 or 16 channels wide) starts at Z row 1 - dy, so the
 //     blocks dy = +1, 0, -1 are whole-row offsets (the rest of M is unused);
 //     the zero rows keep every pixel outside the tile out of the sum.
-//   B (N = 3 CI + 16): the three dx-shifted boxes of the input halo (the
-//     boxes of k_conv_tc, circular edges rewritten the same way) side by
-//     side, then a block of ones -- whose column gives db from the dy = 0 rows.
-// Thread 0 keeps the boxes of the next two tiles loading into three slots
-// while the MMAs of this one run; at the end the 4 warps read D (warp w: lanes 32 w ..)
-// and write the CTA's partial sums in k_conv_wgrad's layout for k_reduce_rows.
+//   B (N = 3 CI + 16): the three dx-shifted boxes of the input halo side by
+//     side (in the swizzled layout that a TMA box would have), then a block of
+//     ones -- whose column gives db from the dy = 0 rows.
+// Eight warps read the 10 x 18 halo of the next tile into registers (16-byte
+// loads, circular at the image edges) while the MMAs of this one run, and
+// write each chunk to the up to three boxes that hold it; one thread of a ninth
+// warp loads the dz boxes by TMA and issues the MMAs, three slots deep.  As
+// three TMA boxes the input cost 480 of a tile's 608 64-byte box rows, which
+// the SM's TMA unit takes at about 6 cycles each: a 32 -> 32 layer over
+// 64 x 192^2 pixels went from 268 to 152 us.  The MMAs (10 per tile) bound it
+// now.
+// At the end warps 0-3 read D (warp w: lanes 32 w ..) and write the CTA's
+// partial sums in k_conv_wgrad's layout for k_reduce_rows.
 // Every wait is bounded (bit 4 of *err, the partial sums are then zero).
 template <int CI, int CO>
 struct WgTile {
@@ -1162,6 +1169,8 @@ struct WgTile {
     static constexpr int ZROWS = CO == 32 ? 16 : 24;
     static constexpr int ZB = ZROWS * kConvTX * ROWD;
     static constexpr int SLOT = 4 * BOXI + ZB;                // 3 dx boxes, the ones block, Z
+    static constexpr int COPY = 256;                          // threads that copy the input halo
+    static constexpr int CHUNKS = (kConvTY + 2) * (kConvTX + 2) * (CI / 8);   // 16-byte chunks of a 10 x 18 halo
     static constexpr int NSLOT = 3;
     static constexpr int N = 3 * CI + 16;
     static constexpr size_t SMEM = NSLOT * (size_t)SLOT + 1024;
@@ -1182,8 +1191,7 @@ __device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t lbo, u
 }
 
 template <int CI, int CO>
-__global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUtensorMap tin,
-                                                     const __grid_constant__ CUtensorMap tdz,
+__global__ void __launch_bounds__(WgTile<CI, CO>::COPY + 32, 1) k_wgrad_tc(const __grid_constant__ CUtensorMap tdz,
                                                      const __nv_bfloat16* __restrict__ in, float* part, int B,
                                                      int H, int Wd, unsigned int* err) {
     using WT = WgTile<CI, CO>;
@@ -1197,8 +1205,8 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
     __shared__ __align__(8) uint64_t mbar_full[NS];
     __shared__ __align__(8) uint64_t mbar_mma[NS];
     __shared__ uint32_t tmem_base;
-    __shared__ int s_ok;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const bool control = tid == WT::COPY;   // the thread that loads dz and issues the MMAs
     const int tiles_x = (Wd + kConvTX - 1) / kConvTX;
     const int tiles_img = tiles_x * ((H + kConvTY - 1) / kConvTY);
     const int ntiles = tiles_img * B;
@@ -1224,7 +1232,6 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&mbar_mma[s])) : "memory");
         }
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-        s_ok = 1;
     }
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -1239,64 +1246,87 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
         tx0 = (tl % tiles_x) * kConvTX;
         ty0 = (tl / tiles_x) * kConvTY;
     };
-    auto issue_loads = [&](int k) {
-        const int s = k % NS;
+    auto issue_dz = [&](int k) {
+        const int sl = k % NS;
         int b, tx0, ty0;
         tile_xy(k, b, tx0, ty0);
-        const uint32_t slot = sbase + s * WT::SLOT;
-        const uint32_t bar = smem_u32(&mbar_full[s]);   // slot s, (k / NS)-th use
-        mbar_expect_tx(bar, (uint32_t)(3 * WT::BOXI + WT::BOXD));
-#pragma unroll
-        for (int d = 0; d < 3; ++d) tma_load_4d(slot + d * WT::BOXI, &tin, 0, tx0 + d - 1, ty0 - 1, b, bar);
-        tma_load_4d(slot + 4 * WT::BOXI + 2 * kConvTX * ROWD, &tdz, 0, tx0, ty0, b, bar);
+        const uint32_t bar = smem_u32(&mbar_full[sl]);   // slot sl, (k / NS)-th use
+        mbar_expect_tx(bar, (uint32_t)WT::BOXD);
+        tma_load_4d(sbase + sl * WT::SLOT + 4 * WT::BOXI + 2 * kConvTX * ROWD, &tdz, 0, tx0, ty0, b, bar);
     };
-    // thread 0's bookkeeping: loads issued up to tile kl, MMAs committed up to km
+    // this thread's chunks of the halo of tile k: chunk i is 16 bytes q of
+    // pixel (hr, c), image row ty0 + hr - 1, column tx0 + c - 1 (circular)
+    constexpr int HW = kConvTX + 2, NCH = (WT::CHUNKS + WT::COPY - 1) / WT::COPY;
+    uint4 v[NCH];
+    auto load_halo = [&](int k) {
+        int b, tx0, ty0;
+        tile_xy(k, b, tx0, ty0);
+        const long img = (long)b * H * Wd;
+#pragma unroll
+        for (int j = 0; j < NCH; ++j) {
+            const int i = tid + j * WT::COPY;
+            const int q = i % KGI, r = i / KGI;
+            int yy = ty0 + r / HW - 1, xx = tx0 + r % HW - 1;
+            // yy in [-1, H + 8), xx in [-1, Wd + 16]: at most two wraps (grid >= 8)
+            yy += yy < 0 ? H : 0;
+            yy -= yy >= H ? H : 0;
+            yy -= yy >= H ? H : 0;
+            xx += xx < 0 ? Wd : 0;
+            xx -= xx >= Wd ? Wd : 0;
+            xx -= xx >= Wd ? Wd : 0;
+            if (i < WT::CHUNKS) v[j] = *reinterpret_cast<const uint4*>(in + (img + (long)yy * Wd + xx) * CI + q * 8);
+        }
+    };
+    auto store_halo = [&](int k) {
+        unsigned char* slotp = gbase + (k % NS) * WT::SLOT;
+#pragma unroll
+        for (int j = 0; j < NCH; ++j) {
+            const int i = tid + j * WT::COPY;
+            if (i >= WT::CHUNKS) break;
+            const int q = i % KGI, r = i / KGI;
+            const int hr = r / HW, c = r % HW;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {   // box d holds the columns d .. d + 15
+                const int cc = c - d;
+                if (cc < 0 || cc >= kConvTX) continue;
+                const int row = hr * kConvTX + cc;
+                const int pq = ROWI == 64 ? (q ^ ((row >> 1) & 3)) : (q ^ ((row >> 2) & 1));
+                *reinterpret_cast<uint4*>(slotp + d * WT::BOXI + row * ROWI + pq * 16) = v[j];
+            }
+        }
+    };
+    // the control thread's bookkeeping: dz loads issued up to tile kl, MMAs
+    // committed up to km
     int kl = 0, km = -1;
-    if (tid == 0)
-        while (kl < nk && kl < NS - 1) issue_loads(kl++);
+    bool ok = true;
+    if (control && nk > 0) issue_dz(kl++);
+    if (tid < WT::COPY && nk > 0) load_halo(0);
 
     for (int k = 0; k < nk; ++k) {
-        const int s = k % NS;
-        const uint32_t par = (uint32_t)(k / NS) & 1u;
-        int b, tx0, ty0;
-        tile_xy(k, b, tx0, ty0);
-        if (tid == 0 && !mbar_wait_bounded(smem_u32(&mbar_full[s]), par)) s_ok = 0;
-        __syncthreads();
-        if (!s_ok) break;
-        // circular wrap at the image edges: rewrite the zero-filled positions
-        // of the three input boxes (as k_conv_tc)
-        if (tx0 == 0 || ty0 == 0 || tx0 + kConvTX >= Wd || ty0 + kConvTY >= H) {
-            (void)mbar_try_wait(smem_u32(&mbar_full[s]), par);
-            const long img = (long)b * H * Wd;
-            unsigned char* slotp = gbase + s * WT::SLOT;
-            for (int i = tid; i < 3 * (kConvTY + 2) * kConvTX * KGI; i += blockDim.x) {
-                const int q = i % KGI;
-                int r = i / KGI;
-                const int c = r % kConvTX;
-                r /= kConvTX;
-                const int hr = r % (kConvTY + 2);
-                const int d = r / (kConvTY + 2);
-                int yy = ty0 + hr - 1, xx = tx0 + c + d - 1;
-                if (yy >= 0 && yy < H && xx >= 0 && xx < Wd) continue;
-                yy += yy < 0 ? H : 0;
-                yy -= yy >= H ? H : 0;
-                yy -= yy >= H ? H : 0;
-                xx += xx < 0 ? Wd : 0;
-                xx -= xx >= Wd ? Wd : 0;
-                xx -= xx >= Wd ? Wd : 0;
-                const uint4 v = *reinterpret_cast<const uint4*>(in + (img + (long)yy * Wd + xx) * CI + q * 8);
-                const int row = hr * kConvTX + c;
-                const int pq = ROWI == 64 ? (q ^ ((row >> 1) & 3)) : (q ^ ((row >> 2) & 1));
-                *reinterpret_cast<uint4*>(slotp + d * WT::BOXI + row * ROWI + pq * 16) = v;
+        const int sl = k % NS;
+        if (tid < WT::COPY) {
+            // slot sl is free: the control thread waited for the MMAs of tile
+            // k - NS before the last barrier
+            store_halo(k);
+            if (k + 1 < nk) load_halo(k + 1);
+        } else if (control) {
+            if (k + 1 < nk) {   // the slot of tile k + 1
+                ok = k + 1 < NS ||
+                     mbar_wait_bounded(smem_u32(&mbar_mma[(k + 1) % NS]), (uint32_t)((k + 1) / NS - 1) & 1u);
+                if (ok) issue_dz(kl++);
             }
+            ok = ok && mbar_wait_bounded(smem_u32(&mbar_full[sl]), (uint32_t)(k / NS) & 1u);
         }
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-        __syncthreads();
+        if (!__syncthreads_and(ok)) {
+            ok = false;
+            break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-        if (tid == 0) {
+        if (control) {
             constexpr uint32_t idesc = umma_idesc_bf16(128, WT::N) | (1u << 15) | (1u << 16);   // A, B MN-major
-            const uint32_t slot = sbase + s * WT::SLOT;
+            const uint32_t slot = sbase + sl * WT::SLOT;
             const uint32_t z = slot + 4 * WT::BOXI;
 #pragma unroll 1
             for (int rho = 0; rho < kConvTY + 2; ++rho) {
@@ -1310,27 +1340,22 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
                     : "memory");
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                             smem_u32(&mbar_mma[s]))
+                             smem_u32(&mbar_mma[sl]))
                          : "memory");
             km = k;
-            // tile k + NS - 1 goes to the slot of tile k - 1 once the MMAs
-            // that read it are done
-            if (kl < nk) {
-                if (k >= 1 && !mbar_wait_bounded(smem_u32(&mbar_mma[(k - 1) % NS]), (uint32_t)((k - 1) / NS) & 1u))
-                    s_ok = 0;
-                else
-                    issue_loads(kl++);
-            }
         }
     }
     // every MMA complete before the accumulator is read
-    if (tid == 0 && km >= 0 && !mbar_wait_bounded(smem_u32(&mbar_mma[km % NS]), (uint32_t)(km / NS) & 1u)) s_ok = 0;
-    if (tid == 0 && !s_ok) {
-        atomicOr(err, 4u);
-        for (int k = km + 1; k < kl; ++k) mbar_wait_bounded(smem_u32(&mbar_full[k % NS]), (uint32_t)(k / NS) & 1u);
+    if (control) {
+        if (km >= 0 && !mbar_wait_bounded(smem_u32(&mbar_mma[km % NS]), (uint32_t)(km / NS) & 1u)) ok = false;
+        if (!ok) {
+            atomicOr(err, 4u);
+            for (int k = km + 1; k < kl; ++k)
+                mbar_wait_bounded(smem_u32(&mbar_full[k % NS]), (uint32_t)(k / NS) & 1u);
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
+    ok = __syncthreads_and(ok) && nk > 0;
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 
     // D row m = (block i = m / CO: dy = 1 - i, channel co = m % CO); column
@@ -1339,29 +1364,30 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
     float* out = part + (long)blockIdx.x * stride;
     const int m = warp * 32 + lane;
     const int blk = m / CO, co = m % CO;
-    const bool ok = s_ok && nk > 0;
+    if (warp < 4) {
 #pragma unroll 1
-    for (int c0 = 0; c0 < WT::N; c0 += 16) {
-        uint32_t r[16];
-        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (blk > 2) continue;
-        const int dy = 1 - blk;
+        for (int c0 = 0; c0 < WT::N; c0 += 16) {
+            uint32_t r[16];
+            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                  "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                : "r"(taddr));
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+            if (blk > 2) continue;
+            const int dy = 1 - blk;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            const int n = c0 + e;
-            const float v = ok ? __uint_as_float(r[e]) : 0.0f;
-            if (n < 3 * CI) {
-                const int dx = n / CI - 1, ci = n % CI;
-                const int t = (dy + 1) * 3 + (dx + 1);
-                out[((long)co * 9 + t) * CI + ci] = v;
-            } else if (n == 3 * CI && dy == 0) {
-                out[(long)CO * 9 * CI + co] = v;
+            for (int e = 0; e < 16; ++e) {
+                const int n = c0 + e;
+                const float v = ok ? __uint_as_float(r[e]) : 0.0f;
+                if (n < 3 * CI) {
+                    const int dx = n / CI - 1, ci = n % CI;
+                    const int t = (dy + 1) * 3 + (dx + 1);
+                    out[((long)co * 9 + t) * CI + ci] = v;
+                } else if (n == 3 * CI && dy == 0) {
+                    out[(long)CO * 9 * CI + co] = v;
+                }
             }
         }
     }
@@ -1376,13 +1402,12 @@ __global__ void __launch_bounds__(128, 1) k_wgrad_tc(const __grid_constant__ CUt
 template <int CI, int CO>
 cudaError_t launch_wgrad(const __nv_bfloat16* dz, const __nv_bfloat16* in, float* part, int B, int H, int Wd,
                          int grid, unsigned int* err, cudaStream_t st, int* nblk) {
-    CUtensorMap mi, md;
-    cudaError_t e = conv_tensor_map<CI>(&mi, in, B, H, Wd);
-    if (e == cudaSuccess) e = conv_tensor_map<CO>(&md, dz, B, H, Wd, kConvTY);
+    CUtensorMap md;
+    const cudaError_t e = conv_tensor_map<CO>(&md, dz, B, H, Wd, kConvTY);
     if (e != cudaSuccess) return e;
     const long ntiles = (long)((Wd + kConvTX - 1) / kConvTX) * ((H + kConvTY - 1) / kConvTY) * B;
     *nblk = (int)std::max<long>(1, std::min<long>(ntiles, grid));
-    return launch_k(k_wgrad_tc<CI, CO>, *nblk, 128, WgTile<CI, CO>::SMEM, st, false, mi, md, in, part, B, H, Wd,
+    return launch_k(k_wgrad_tc<CI, CO>, *nblk, WgTile<CI, CO>::COPY + 32, WgTile<CI, CO>::SMEM, st, false, md, in, part, B, H, Wd,
                     err);
 }
 
