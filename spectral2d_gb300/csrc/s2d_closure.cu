@@ -221,10 +221,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 constexpr int kMbarSpinLimit = 1 << 22;
 
 // Shared-memory matrix descriptor of a K-major operand stored with the
-// 32- or 64-byte swizzle (rows of ROWB = 32 or 64 bytes, 8-row atoms of
+// 32-, 64- or 128-byte swizzle (rows of ROWB bytes, 8-row atoms of
 // 8 * ROWB bytes, 16-byte chunk c of row r stored at chunk c ^ ((r >> s) & m)
-// with s = 2, m = 1 for 32 B and s = 1, m = 3 for 64 B -- the layout TMA
-// writes with CU_TENSOR_MAP_SWIZZLE_32B / _64B): sbo = the atom stride; a K
+// with s = 2, m = 1 for 32 B, s = 1, m = 3 for 64 B and s = 0, m = 7 for 128 B
+// -- the layout TMA writes with CU_TENSOR_MAP_SWIZZLE_32B / _64B / _128B): sbo = the atom stride; a K
 // offset within a row is added to the start address.
 template <int ROWB>
 __device__ __forceinline__ uint64_t umma_desc_sw(uint32_t saddr) {
@@ -232,7 +232,7 @@ __device__ __forceinline__ uint64_t umma_desc_sw(uint32_t saddr) {
     d |= (uint64_t)1 << 16;                                    // leading offset: unused for this layout
     d |= (uint64_t)(((8u * ROWB) >> 4) & 0x3FFFu) << 32;       // stride offset: one 8-row atom
     d |= (uint64_t)1 << 46;                                    // descriptor version of the sm_100 family
-    d |= (uint64_t)(ROWB == 64 ? 4 : 6) << 61;                 // 64-byte or 32-byte swizzle
+    d |= (uint64_t)(ROWB == 128 ? 2 : ROWB == 64 ? 4 : 6) << 61;   // 128-, 64- or 32-byte swizzle
     return d;
 }
 
@@ -626,7 +626,9 @@ cudaError_t conv_tensor_map(CUtensorMap* map, const __nv_bfloat16* act, int B, i
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(act), dims, strides,
                            box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           KC == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                           KC == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                           : KC == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                      : CU_TENSOR_MAP_SWIZZLE_32B,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
@@ -651,7 +653,8 @@ cudaError_t launch_conv(const __nv_bfloat16* in, const __nv_bfloat16* W, const f
 // All six layers of the network in one persistent launch, for the forward
 // passes that keep no pre-activations (the LES closure term, inference).
 //
-// Images carry a one-pixel circular frame: [B][H + 2][Wd + 2][KC], pixel
+// Images carry a one-pixel circular frame: [B][H + 2][Wd + 2][KC] (an odd Wd + 2
+// padded by one pixel, which no output reads), pixel
 // (y, x) at (y + 1, x + 1), frame row 0 = image row H - 1, frame row H + 1 =
 // image row 0, likewise the columns and the corners.  A layer's epilogue
 // writes each border pixel into the frame as well (up to four copies), so
@@ -661,16 +664,21 @@ cudaError_t launch_conv(const __nv_bfloat16* in, const __nv_bfloat16* W, const f
 // of them are resident).
 //
 // The three column taps dx of a row of taps dy go side by side into the
-// MMA's N dimension: for a box of 10 x 16 pixels (one TMA box, the tile's
-// 8 x 14 outputs and their halo) D[m, (dx, n)] = sum over dy and channels of
-// box pixel m + 16 (dy + 1) times W[n, (dy, dx), :], so a tile is 3 KC / 16
-// MMAs of N = 3 NC (not 9 KC / 16 of N = NC, each of which streams the same
-// 4 KB of activations from shared memory for only 32 columns), and output
-// pixel m takes column block dx at pixel m + dx - 1, a warp shuffle.
+// MMA's N dimension, and a row of the MMA is P = 1 pixel or a pair (P = 2): for
+// a box of 10 x 16 rows of P pixels (one TMA box, the tile's 8 x (16 P - 2)
+// outputs and their halo) and pixel par of them, D_par[m, (dx, n)] = sum over dy
+// and channels of pixel par of box row m + 16 (dy + 1) times W[n, (dy, dx), :],
+// so a tile is P x 3 KC / 16 MMAs of N = 3 NC (not 9 KC / 16 of N = NC, each of
+// which streams the same 4 KB of activations from shared memory for only 32
+// columns).  An output pixel sums column block dx at the pixel dx beside it:
+// its pair's other pixel, or that of the next row, a warp shuffle.  Pairs
+// because the SM's TMA unit takes a box row of 64 bytes (one pixel) in no less
+// time than one of 128: tiles of pixels hold the pipeline at 895 cycles each,
+// 0.80 of the 1.08 ms of 32 x 384^2 pixels (0.87 ms with pairs).
 // One CTA per SM (the cooperative limit): warp 17 issues the TMA loads of
-// the boxes into four slots, warp 16 the MMAs of a tile into one of four
-// tensor-memory accumulators (descriptors precomputed per slot: a row of
-// taps is an offset of the start address), and two groups of eight warps
+// the boxes into four slots, warp 16 the MMAs of a tile into one of 4 / P
+// tensor-memory accumulators of P parities (a row of taps or a parity is an
+// offset of the start address), and two groups of eight warps
 // take alternate tiles: read the accumulator, release it (mbarrier), sum the
 // taps, apply bias and GELU and store, while the MMAs of the following tiles
 // run.  The roles meet only at mbarriers: full (slot landed), mmad (its MMAs
@@ -678,24 +686,30 @@ cudaError_t launch_conv(const __nv_bfloat16* in, const __nv_bfloat16* W, const f
 // Every wait is bounded: a wait that runs out sets bit 4 of *err and
 // the abort flag, the CTA skips the rest (after bounded waits for its copies
 // and MMAs in flight) and frees its tensor memory.
+__host__ __device__ inline int net_pitch(int Wd) { return (Wd + 3) & ~1; }   // pixels of a framed row, even
 constexpr int kNetGroups = 2;                    // epilogue groups of 8 warps (tile i: group i % 2)
-// Accumulators = box slots: tile i uses slot and accumulator i % 4, and one
-// commit per tile (mmad) tells the epilogue the accumulator is ready and the
-// producer the slot is free (a tcgen05.commit costs the tensor pipe about as
-// much as three of these MMAs, so there is one per tile, not two).
-constexpr int kNetAcc = 4;
+// Tile i uses box slot i % 4 and accumulator i % (4 / P); one commit per tile (mmad of
+// the slot) tells the epilogue the accumulator is ready and the producer the
+// slot is free (a tcgen05.commit costs the tensor pipe about as much as three
+// of these MMAs, so there is one per tile, not two).
 constexpr int kNetEpiWarps = 8 * kNetGroups;     // warps 0-15
 constexpr int kNetMmaWarp = kNetEpiWarps;        // warp 16
 constexpr int kNetProdWarp = kNetEpiWarps + 1;   // warp 17
 constexpr int kNetThreads = 32 * (kNetEpiWarps + 2);
-constexpr int kNetAccCols = 128;                 // 3 * 32 columns used
-constexpr int kNetTmemCols = kNetAccCols * kNetAcc;
-constexpr int kNetOutH = 8, kNetOutW = 14;       // output tile
-constexpr int kNetBoxRows = kNetOutH + 2, kNetBoxW = kNetOutW + 2;   // its halo box: M = 8 x 16 = 128 pixels
-constexpr int kNetSlots = kNetAcc;
-constexpr int kNetSlotBytes = kNetBoxRows * kNetBoxW * 64;   // one box of 32-channel pixels
+constexpr int kNetParCols = 128;                 // of one pixel parity: 3 * 32 columns used
+constexpr int kNetTmemCols = 4 * kNetParCols;
+constexpr int kNetOutH = 8, kNetBoxRows = kNetOutH + 2;      // rows of a tile and of its halo box
+constexpr int kNetBoxW = 16;                                 // MMA rows (P pixels each) of a box row: M = 8 x 16
+template <int P>
+constexpr int kNetOutW = kNetBoxW * P - 2;                   // output columns of a tile
+template <int P>
+constexpr int kNetAcc = 4 / P;                               // accumulators of P parities
+constexpr int kNetSlots = 4;
+template <int P>
+constexpr int kNetSlotBytes = kNetBoxRows * kNetBoxW * 64 * P;   // one box of 32-channel pixels
 constexpr int kNetWBytes = 3 * 96 * 4 * 16;                  // B operands of the three rows of taps
-constexpr size_t kNetSmem = (size_t)kNetSlots * kNetSlotBytes + kNetWBytes + 1024;
+template <int P>
+constexpr size_t kNetSmem = (size_t)kNetSlots * kNetSlotBytes<P> + kNetWBytes + 1024;
 
 struct NetArgs {
     const __nv_bfloat16* W[kLayers];   // BF16 working weights W[n][t][k]
@@ -710,8 +724,8 @@ struct NetArgs {
 
 struct NetShared {
     uint64_t full[kNetSlots];   // the boxes of a slot have landed
-    uint64_t mmad[kNetAcc];     // the MMAs of the tile in slot / accumulator are complete
-    uint64_t accfree[kNetAcc];  // the 8 warps of its epilogue group have read an accumulator
+    uint64_t mmad[kNetSlots];   // the MMAs of the tile in the slot are complete
+    uint64_t accfree[4];        // the 8 warps of its epilogue group have read an accumulator
     uint32_t tmem;
     int abort;
     float bias[32];
@@ -758,7 +772,7 @@ __device__ __forceinline__ bool net_grid_wait(const unsigned int* bar, unsigned 
 // A layer's weights as the B operands of the three rows of taps: for row dy,
 // column group g = (dx, 8 output channels), the input channels K-major in core
 // matrices; and its biases.  At most two 16-byte pieces per thread.
-template <int KC, int NC>
+template <int P, int KC, int NC>
 __device__ __forceinline__ void net_stage_weights(const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
                                                   NetShared& sh, unsigned char* gbase) {
     constexpr int KG = KC / 8, N = 3 * NC, NG = N / 8, CORE = 128;
@@ -772,7 +786,7 @@ __device__ __forceinline__ void net_stage_weights(const __nv_bfloat16* __restric
         const int t = dyi * 3 + dxi;
         const uint4 v = *reinterpret_cast<const uint4*>(W + ((long)n * 9 + t) * KC + kg * 8);
         const int off = ((dyi * NG + g) * KG + kg) * CORE + nl * 16;
-        *reinterpret_cast<uint4*>(gbase + kNetSlots * kNetSlotBytes + off) = v;
+        *reinterpret_cast<uint4*>(gbase + kNetSlots * kNetSlotBytes<P> + off) = v;
     }
     if ((int)threadIdx.x < NC) sh.bias[threadIdx.x] = bias[threadIdx.x];
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -781,11 +795,11 @@ __device__ __forceinline__ void net_stage_weights(const __nv_bfloat16* __restric
 // One layer over this CTA's tiles (tile blockIdx.x + k gridDim.x), its weights
 // staged; irun is the CTA's running tile count over all layers, which fixes
 // every slot, accumulator and barrier phase.
-template <int KC, int NC, bool LAST>
+template <int P, int KC, int NC, bool LAST>
 __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16* out, float* yout, const NetArgs& a,
                                           NetShared& sh, uint32_t sbase, int& irun) {
     constexpr int KG = KC / 8;                 // 8-channel groups of a pixel
-    constexpr int ROWB = KC * 2;               // bytes of one pixel
+    constexpr int ROWB = KC * 2 * P;           // bytes of an MMA row: a pixel or a pair
     constexpr int BOX = kNetBoxRows * kNetBoxW * ROWB;
     constexpr int N = 3 * NC;                  // the MMA's columns: (dx, output channel)
     constexpr int NG = N / 8;                  // 8-column groups
@@ -793,11 +807,11 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16*
     constexpr int WGROUP = KG * CORE;          // 8 columns x all input channels
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int H = a.H, Wd = a.Wd;
-    const int tiles_x = (Wd + kNetOutW - 1) / kNetOutW;
+    const int tiles_x = (Wd + kNetOutW<P> - 1) / kNetOutW<P>;
     const int tiles_img = tiles_x * ((H + kNetOutH - 1) / kNetOutH);
     const int ntiles = tiles_img * a.B;
     const int nk = (int)blockIdx.x < ntiles ? (ntiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-    const uint32_t bw = sbase + kNetSlots * kNetSlotBytes;
+    const uint32_t bw = sbase + kNetSlots * kNetSlotBytes<P>;
     volatile int* abort = &sh.abort;
 
     // tile k: output rows [oy0, oy0 + 8), columns [ox0, ox0 + 14); its box is
@@ -807,7 +821,7 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16*
         const int tile = (int)blockIdx.x + k * (int)gridDim.x;
         b = tile / tiles_img;
         const int tl = tile - b * tiles_img;
-        ox0 = (tl % tiles_x) * kNetOutW;
+        ox0 = (tl % tiles_x) * kNetOutW<P>;
         oy0 = (tl / tiles_x) * kNetOutH;
     };
     const int i0 = irun;
@@ -833,7 +847,7 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16*
                 tile_xy(kl, b, ox0, oy0);
                 const uint32_t bar = smem_u32(&sh.full[s]);
                 mbar_expect_tx(bar, (uint32_t)BOX);
-                tma_load_4d(sbase + s * kNetSlotBytes, tin, 0, ox0, oy0, b, bar);
+                tma_load_4d(sbase + s * kNetSlotBytes<P>, tin, 0, ox0 / P, oy0, b, bar);
             }
             if (!ok) {
                 fail();
@@ -855,32 +869,38 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16*
             int km = -1;
             bool ok = true;
             for (int k = 0; k < nk; ++k) {
-                const int i = i0 + k, s = i % kNetSlots, acc = i % kNetAcc;
+                const int i = i0 + k, s = i % kNetSlots, acc = i % kNetAcc<P>;
                 if (!(ok = net_wait(smem_u32(&sh.full[s]), (uint32_t)(i / kNetSlots) & 1u, abort))) break;
-                if (i >= kNetAcc &&
-                    !(ok = net_wait(smem_u32(&sh.accfree[acc]), (uint32_t)(i / kNetAcc - 1) & 1u, abort)))
+                if (i >= kNetAcc<P> &&
+                    !(ok = net_wait(smem_u32(&sh.accfree[acc]), (uint32_t)(i / kNetAcc<P> - 1) & 1u, abort)))
                     break;
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-                const uint64_t ad0 = umma_desc_sw<ROWB>(sbase + s * kNetSlotBytes);
-                const uint32_t dacc = sh.tmem + (uint32_t)(acc * kNetAccCols);
+                const uint64_t ad0 = umma_desc_sw<ROWB>(sbase + s * kNetSlotBytes<P>);
+                const uint32_t dacc = sh.tmem + (uint32_t)(acc * P * kNetParCols);
 #pragma unroll
-                for (int dyi = 0; dyi < 3; ++dyi) {
+                for (int par = 0; par < P; ++par) {
 #pragma unroll
-                    for (int j = 0; j < KC / 16; ++j) {
-                        // box rows dyi .. dyi + 7 (whole 8-pixel atoms); start
-                        // addresses advance in 16-byte units in the low field
-                        const uint64_t ad = ad0 + (uint64_t)((dyi * kNetBoxW * ROWB + j * 32) >> 4);
-                        const uint64_t bd = bd0 + (uint64_t)((dyi * NG * WGROUP + j * 2 * CORE) >> 4);
-                        asm volatile(
-                            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(dacc),
-                            "l"(ad), "l"(bd), "r"(idesc), "r"((dyi | j) ? 1u : 0u)
-                            : "memory");
+                    for (int dyi = 0; dyi < 3; ++dyi) {
+#pragma unroll
+                        for (int j = 0; j < KC / 16; ++j) {
+                            // box rows dyi .. dyi + 7 (whole 8-row atoms), the
+                            // pairs' pixel par; start addresses advance in
+                            // 16-byte units in the low field
+                            const uint64_t ad =
+                                ad0 + (uint64_t)((dyi * kNetBoxW * ROWB + par * KC * 2 + j * 32) >> 4);
+                            const uint64_t bd = bd0 + (uint64_t)((dyi * NG * WGROUP + j * 2 * CORE) >> 4);
+                            asm volatile(
+                                "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                                " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+                                    dacc + (uint32_t)(par * kNetParCols)),
+                                "l"(ad), "l"(bd), "r"(idesc), "r"((dyi | j) ? 1u : 0u)
+                                : "memory");
+                        }
                     }
                 }
                 asm volatile(
                     "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                        smem_u32(&sh.mmad[acc]))
+                        smem_u32(&sh.mmad[s]))
                     : "memory");
                 km = k;
             }
@@ -888,20 +908,20 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16*
                 fail();
                 if (km >= 0) {
                     const int i = i0 + km;
-                    mbar_wait_bounded(smem_u32(&sh.mmad[i % kNetAcc]), (uint32_t)(i / kNetAcc) & 1u);
+                    mbar_wait_bounded(smem_u32(&sh.mmad[i % kNetSlots]), (uint32_t)(i / kNetSlots) & 1u);
                 }
             }
         }
     } else {
         // ---- epilogue warps: group g = w / 8 takes the tiles with i % 2 == g;
-        // warp w reads accumulator lanes 32 (w % 4) .. + 31 (box pixels m: row
-        // m / 16, column m % 16) and, of each tap column dx, the output
-        // channels 16 ((w % 8) / 4) .. + 15.  Output pixel m sums tap dx
-        // evaluated at box pixel m + dx: a shuffle within the 16 lanes of its
-        // row; box columns 1 .. 14 are the tile's outputs.
+        // warp w reads accumulator lanes 32 (w % 4) .. + 31 and, of each tap
+        // column dx, the output channels 16 ((w % 8) / 4) .. + 15.  An output
+        // pixel sums tap dx evaluated at the box pixel dx beside it: a shuffle
+        // within the 16 lanes of its box row; box pixels 1 .. 16 P - 2 of a row
+        // are the tile's outputs.
         const int grp = warp >> 3, quarter = warp & 3, half = (warp >> 2) & 1;
         const bool cols = half * 16 < NC;   // warp-uniform
-        const long fw = Wd + 2;
+        const long fw = net_pitch(Wd);
         // this thread's 16 biases in registers (shared-memory reads per tile
         // would compete with the tensor core's operand reads)
         f32x2 bv[8];
@@ -909,70 +929,88 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16*
         for (int e = 0; e < 8; ++e)
             bv[e] = cols ? pk2(sh.bias[half * 16 + 2 * e], sh.bias[half * 16 + 2 * e + 1]) : 0ull;
         for (int k = (grp - (i0 & 1) + 2) & 1; k < nk; k += kNetGroups) {
-            const int i = i0 + k, acc = i % kNetAcc;
-            if (!net_wait(smem_u32(&sh.mmad[acc]), (uint32_t)(i / kNetAcc) & 1u, abort)) {
+            const int i = i0 + k, acc = i % kNetAcc<P>;
+            if (!net_wait(smem_u32(&sh.mmad[i % kNetSlots]), (uint32_t)(i / kNetSlots) & 1u, abort)) {
                 fail();
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-            uint32_t r[3][16];
-            if (cols) {
-#pragma unroll
-                for (int dxi = 0; dxi < 3; ++dxi) {
-                    const uint32_t taddr = sh.tmem + ((uint32_t)(quarter * 32) << 16) +
-                                           (uint32_t)(acc * kNetAccCols + dxi * NC + half * 16);
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,"
-                        "%15}, [%16];\n"
-                        : "=r"(r[dxi][0]), "=r"(r[dxi][1]), "=r"(r[dxi][2]), "=r"(r[dxi][3]), "=r"(r[dxi][4]),
-                          "=r"(r[dxi][5]), "=r"(r[dxi][6]), "=r"(r[dxi][7]), "=r"(r[dxi][8]), "=r"(r[dxi][9]),
-                          "=r"(r[dxi][10]), "=r"(r[dxi][11]), "=r"(r[dxi][12]), "=r"(r[dxi][13]), "=r"(r[dxi][14]),
-                          "=r"(r[dxi][15])
-                        : "r"(taddr));
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-            }
-            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&sh.accfree[acc]));
-            if (!cols) continue;
-
             int b, ox0, oy0;
             tile_xy(k, b, ox0, oy0);
+            // accumulator row m: pixel or pair m % 16 of box row m / 16
             const int m = quarter * 32 + lane;
-            const int c = m % kNetBoxW;
-            const int y = oy0 + m / kNetBoxW, x = ox0 - 1 + c;
-            const bool valid = c >= 1 && c <= kNetOutW && y < H && x < Wd;
-            auto pair = [](uint32_t p, uint32_t q) { return pk2(__uint_as_float(p), __uint_as_float(q)); };
-            f32x2 z[8];
+            const int pi = m % kNetBoxW;
+            const int y = oy0 + m / kNetBoxW, x = ox0 - 1 + P * pi;   // of the row's first pixel
+            // CH channels at a time (registers)
+            constexpr int CH = 16 / P;
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const f32x2 up = pair(__shfl_up_sync(0xffffffffu, r[0][2 * e], 1, kNetBoxW),
-                                      __shfl_up_sync(0xffffffffu, r[0][2 * e + 1], 1, kNetBoxW));
-                const f32x2 dn = pair(__shfl_down_sync(0xffffffffu, r[2][2 * e], 1, kNetBoxW),
-                                      __shfl_down_sync(0xffffffffu, r[2][2 * e + 1], 1, kNetBoxW));
-                z[e] = add2(add2(add2(up, pair(r[1][2 * e], r[1][2 * e + 1])), dn), bv[e]);
-            }
-            if (!valid) continue;
-            if (LAST) {
-                if (half == 0) yout[((long)b * H + y) * Wd + x] = unpk2(z[0]).x;
-            } else {
-                uint32_t v[8];
-                gelu_pack<8>(z, v);
-                const uint4 lo = make_uint4(v[0], v[1], v[2], v[3]), hi = make_uint4(v[4], v[5], v[6], v[7]);
-                // the pixel and its copies in the frame
-                const long img = (long)b * (H + 2) * fw;
-                const int wy = y == 0 ? H + 1 : (y == H - 1 ? 0 : -1);
-                const int wx = x == 0 ? Wd + 1 : (x == Wd - 1 ? 0 : -1);
-                auto put = [&](int fy, int fx) {
-                    uint4* p = reinterpret_cast<uint4*>(out + (img + fy * fw + fx) * 32 + half * 16);
-                    p[0] = lo;
-                    p[1] = hi;
-                };
-                put(y + 1, x + 1);
-                if (wy >= 0) put(wy, x + 1);
-                if (wx >= 0) put(y + 1, wx);
-                if (wy >= 0 && wx >= 0) put(wy, wx);
+            for (int qq = 0; qq < P; ++qq) {
+                uint32_t r[P][3][CH];
+                if (cols) {
+#pragma unroll
+                    for (int par = 0; par < P; ++par)
+#pragma unroll
+                        for (int dxi = 0; dxi < 3; ++dxi) {
+                            const uint32_t taddr =
+                                sh.tmem + ((uint32_t)(quarter * 32) << 16) +
+                                (uint32_t)((acc * P + par) * kNetParCols + dxi * NC + half * 16 + qq * CH);
+#pragma unroll
+                            for (int c8 = 0; c8 < CH; c8 += 8)
+                                asm volatile(
+                                    "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                                    : "=r"(r[par][dxi][c8]), "=r"(r[par][dxi][c8 + 1]), "=r"(r[par][dxi][c8 + 2]),
+                                      "=r"(r[par][dxi][c8 + 3]), "=r"(r[par][dxi][c8 + 4]),
+                                      "=r"(r[par][dxi][c8 + 5]), "=r"(r[par][dxi][c8 + 6]),
+                                      "=r"(r[par][dxi][c8 + 7])
+                                    : "r"(taddr + (uint32_t)c8));
+                        }
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                }
+                if (qq == P - 1) {
+                    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&sh.accfree[acc]));
+                }
+                if (!cols) continue;
+                auto pair = [](uint32_t p, uint32_t q) { return pk2(__uint_as_float(p), __uint_as_float(q)); };
+                f32x2 z[P][CH / 2];
+#pragma unroll
+                for (int e = 0; e < CH / 2; ++e) {
+                    const f32x2 up = pair(__shfl_up_sync(0xffffffffu, r[P - 1][0][2 * e], 1, kNetBoxW),
+                                          __shfl_up_sync(0xffffffffu, r[P - 1][0][2 * e + 1], 1, kNetBoxW));
+                    const f32x2 dn = pair(__shfl_down_sync(0xffffffffu, r[0][2][2 * e], 1, kNetBoxW),
+                                          __shfl_down_sync(0xffffffffu, r[0][2][2 * e + 1], 1, kNetBoxW));
+                    auto own = [&](int par, int dxi) { return pair(r[par][dxi][2 * e], r[par][dxi][2 * e + 1]); };
+                    const f32x2 bias = bv[qq * (CH / 2) + e];
+                    z[0][e] = add2(add2(add2(up, own(0, 1)), P == 2 ? own(P - 1, 2) : dn), bias);
+                    if (P == 2) z[P - 1][e] = add2(add2(add2(own(0, 0), own(P - 1, 1)), dn), bias);
+                }
+#pragma unroll
+                for (int par = 0; par < P; ++par) {
+                    const int px = x + par, c = P * pi + par;   // box pixels 1 .. 16 P - 2 are outputs
+                    if (c < 1 || c > kNetOutW<P> || y >= H || px >= Wd) continue;
+                    if (LAST) {
+                        if (half == 0 && qq == 0) yout[((long)b * H + y) * Wd + px] = unpk2(z[par][0]).x;
+                    } else {
+                        uint32_t v[CH / 2];
+                        gelu_pack<CH / 2>(z[par], v);
+                        // the pixel and its copies in the frame
+                        const long img = (long)b * (H + 2) * fw;
+                        const int wy = y == 0 ? H + 1 : (y == H - 1 ? 0 : -1);
+                        const int wx = px == 0 ? Wd + 1 : (px == Wd - 1 ? 0 : -1);
+                        auto put = [&](int fy, int fx) {
+                            uint4* q = reinterpret_cast<uint4*>(out + (img + fy * fw + fx) * 32 + half * 16 + qq * CH);
+#pragma unroll
+                            for (int c8 = 0; c8 < CH / 8; ++c8)
+                                q[c8] = make_uint4(v[4 * c8], v[4 * c8 + 1], v[4 * c8 + 2], v[4 * c8 + 3]);
+                        };
+                        put(y + 1, px + 1);
+                        if (wy >= 0) put(wy, px + 1);
+                        if (wx >= 0) put(y + 1, wx);
+                        if (wy >= 0 && wx >= 0) put(wy, wx);
+                    }
+                }
+                __syncwarp();
             }
         }
         // this layer's stores are read by the next layer's TMA (async proxy)
@@ -981,6 +1019,7 @@ __device__ __forceinline__ void net_layer(const CUtensorMap* tin, __nv_bfloat16*
     irun = i0 + nk;
 }
 
+template <int P>
 __global__ void __launch_bounds__(kNetThreads, 1) k_net_fwd(const __grid_constant__ CUtensorMap m_in,
                                                           const __grid_constant__ CUtensorMap m_a0,
                                                           const __grid_constant__ CUtensorMap m_a1, NetArgs a) {
@@ -999,9 +1038,9 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_fwd(const __grid_constan
     if (tid == 0) {
         for (int s = 0; s < kNetSlots; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&sh.full[s])) : "memory");
-        }
-        for (int s = 0; s < kNetAcc; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&sh.mmad[s])) : "memory");
+        }
+        for (int s = 0; s < kNetAcc<P>; ++s) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&sh.accfree[s])),
                          "r"(kNetEpiWarps / kNetGroups)
                          : "memory");
@@ -1028,15 +1067,15 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_fwd(const __grid_constan
         __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     };
-    before_layer([&] { net_stage_weights<16, 32>(a.W[0], a.bias[0], sh, gbase); }, true);
-    net_layer<16, 32, false>(&m_in, a.act[0], nullptr, a, sh, sbase, irun);
+    before_layer([&] { net_stage_weights<P, 16, 32>(a.W[0], a.bias[0], sh, gbase); }, true);
+    net_layer<P, 16, 32, false>(&m_in, a.act[0], nullptr, a, sh, sbase, irun);
 #pragma unroll 1
     for (int l = 1; l < kLayers - 1; ++l) {
-        before_layer([&] { net_stage_weights<32, 32>(a.W[l], a.bias[l], sh, gbase); }, false);
-        net_layer<32, 32, false>(l & 1 ? &m_a0 : &m_a1, a.act[l & 1], nullptr, a, sh, sbase, irun);
+        before_layer([&] { net_stage_weights<P, 32, 32>(a.W[l], a.bias[l], sh, gbase); }, false);
+        net_layer<P, 32, 32, false>(l & 1 ? &m_a0 : &m_a1, a.act[l & 1], nullptr, a, sh, sbase, irun);
     }
-    before_layer([&] { net_stage_weights<32, 16>(a.W[kLayers - 1], a.bias[kLayers - 1], sh, gbase); }, false);
-    net_layer<32, 16, true>(&m_a0, nullptr, a.y, a, sh, sbase, irun);
+    before_layer([&] { net_stage_weights<P, 32, 16>(a.W[kLayers - 1], a.bias[kLayers - 1], sh, gbase); }, false);
+    net_layer<P, 32, 16, true>(&m_a0, nullptr, a.y, a, sh, sbase, irun);
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
     if (warp == kNetMmaWarp)
@@ -1052,7 +1091,7 @@ __global__ void __launch_bounds__(kNetThreads, 1) k_net_fwd(const __grid_constan
 // Framed copy of B images [B][H][Wd][16] (the layer-1 input written
 // unframed): one thread per framed pixel and 16-byte half.
 __global__ void k_frame16(const __nv_bfloat16* __restrict__ x, int B, int H, int Wd, __nv_bfloat16* xf) {
-    const long fw = Wd + 2, fh = H + 2;
+    const long fw = net_pitch(Wd), fh = H + 2;
     const long n = (long)B * fh * fw * 2;
     for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const int q = (int)(i & 1);
@@ -1974,13 +2013,15 @@ int refresh_all(s2d_cnn* c) {
 
 int ensure_net_buffers(s2d_cnn* c) {
     if (c->netbar) return S2D_OK;
-    const size_t fp = (size_t)c->maxB * (c->H + 2) * (c->Wd + 2);
-    C_CUDA(cudaFuncSetAttribute(k_net_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNetSmem));
-    int occ = 0;
-    C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_net_fwd, kNetThreads, kNetSmem));
-    if (occ < 1) return cerr(S2D_ERR_UNSUPPORTED, "the fused network kernel does not fit on an SM");
-    occ = 1;   // one CTA per SM by design (its TMEM columns, the launch bound)
-    c->net_grid = occ * c->sms;
+    const size_t fp = (size_t)c->maxB * (c->H + 2) * net_pitch(c->Wd);
+    const auto A = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    C_CUDA(cudaFuncSetAttribute(k_net_fwd<1>, A, (int)kNetSmem<1>));
+    C_CUDA(cudaFuncSetAttribute(k_net_fwd<2>, A, (int)kNetSmem<2>));
+    int occ1 = 0, occ2 = 0;
+    C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, k_net_fwd<1>, kNetThreads, kNetSmem<1>));
+    C_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, k_net_fwd<2>, kNetThreads, kNetSmem<2>));
+    if (occ1 < 1 || occ2 < 1) return cerr(S2D_ERR_UNSUPPORTED, "the fused network kernel does not fit on an SM");
+    c->net_grid = c->sms;   // one CTA per SM by design (its TMEM columns, the launch bound)
     bool ok = cudaMalloc(&c->X0f, fp * 16 * sizeof(__nv_bfloat16)) == cudaSuccess &&
               cudaMemset(c->X0f, 0, fp * 16 * sizeof(__nv_bfloat16)) == cudaSuccess &&
               cudaMalloc(&c->F[0], fp * 32 * sizeof(__nv_bfloat16)) == cudaSuccess &&
@@ -2000,18 +2041,13 @@ int ensure_net_buffers(s2d_cnn* c) {
 
 // Inference forward of B images in one launch (k_net_fwd); the layer-1 input
 // is in X0f already framed (k_cl_xinv writes it so) or framed here from X0.
-int forward_fused(s2d_cnn* c, int B, bool input_framed) {
-    int r = ensure_net_buffers(c);
-    if (r != S2D_OK) return r;
+template <int P>
+int launch_net(s2d_cnn* c, int B) {
     const int H = c->H, Wd = c->Wd;
-    if (!input_framed) {
-        k_frame16<<<nblocks((long)B * (H + 2) * (Wd + 2) * 2, 256), 256, 0, c->stream>>>(c->X0, B, H, Wd, c->X0f);
-        C_CUDA(cudaGetLastError());
-    }
     CUtensorMap m_in, m_a0, m_a1;
-    C_CUDA(conv_tensor_map<16>(&m_in, c->X0f, B, H + 2, Wd + 2));
-    C_CUDA(conv_tensor_map<32>(&m_a0, c->F[0], B, H + 2, Wd + 2));
-    C_CUDA(conv_tensor_map<32>(&m_a1, c->F[1], B, H + 2, Wd + 2));
+    C_CUDA(conv_tensor_map<16 * P>(&m_in, c->X0f, B, H + 2, net_pitch(Wd) / P));
+    C_CUDA(conv_tensor_map<32 * P>(&m_a0, c->F[0], B, H + 2, net_pitch(Wd) / P));
+    C_CUDA(conv_tensor_map<32 * P>(&m_a1, c->F[1], B, H + 2, net_pitch(Wd) / P));
     NetArgs a{};
     for (int l = 0; l < kLayers; ++l) {
         a.W[l] = c->Wb[l];
@@ -2026,20 +2062,37 @@ int forward_fused(s2d_cnn* c, int B, bool input_framed) {
     a.H = H;
     a.Wd = Wd;
     a.stall = c->net_stall ? 1 : 0;
-    const long ntiles = (long)((Wd + kNetOutW - 1) / kNetOutW) * ((H + kNetOutH - 1) / kNetOutH) * B;
+    const long ntiles = (long)((Wd + kNetOutW<P> - 1) / kNetOutW<P>) * ((H + kNetOutH - 1) / kNetOutH) * B;
     const int grid = (int)std::min<long>(ntiles, c->net_grid);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kNetThreads);
-    cfg.dynamicSmemBytes = kNetSmem;
+    cfg.dynamicSmemBytes = kNetSmem<P>;
     cfg.stream = c->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    C_CUDA(cudaLaunchKernelEx(&cfg, k_net_fwd, m_in, m_a0, m_a1, a));
+    C_CUDA(cudaLaunchKernelEx(&cfg, k_net_fwd<P>, m_in, m_a0, m_a1, a));
     return S2D_OK;
+}
+
+int forward_fused(s2d_cnn* c, int B, bool input_framed) {
+    int r = ensure_net_buffers(c);
+    if (r != S2D_OK) return r;
+    const int H = c->H, Wd = c->Wd;
+    if (!input_framed) {
+        k_frame16<<<nblocks((long)B * (H + 2) * net_pitch(Wd) * 2, 256), 256, 0, c->stream>>>(c->X0, B, H, Wd, c->X0f);
+        C_CUDA(cudaGetLastError());
+    }
+    // Pixel pairs need half the box rows, but their tiles are twice as large:
+    // with few tiles per SM the last round's cost more.  us per LES step, tiles
+    // of pixels / of pairs: 128^2 (2.2 small tiles per SM) 80.5 / 84.0, 192^2 (5)
+    // 98.3 / 100.4, 216^2 (6.5) 114.1 / 109.1, 256^2 114.8 / 115.5, 288^2 133 / 129,
+    // 512^2 257 / 240; 32 runs of 256^2 1656 / 1396.  Both give the same bits.
+    const long small = (long)((Wd + kNetOutW<1> - 1) / kNetOutW<1>) * ((H + kNetOutH - 1) / kNetOutH) * B;
+    return small > 6L * c->sms ? launch_net<2>(c, B) : launch_net<1>(c, B);
 }
 
 // forward of the batch in X0 (B images); the pre-activations z are kept only

@@ -489,3 +489,20 @@ def test_pre_activations_far_from_zero_vs_oracle(S, scale):
     assert np.abs(z).max() > 12.5
     assert _rel(Z[..., :co], _bf(z)) < 1e-3
     assert _rel(A[1][..., :co], _bf(CO.gelu(z))) < 1e-3
+
+
+@pytest.mark.parametrize("grid, B", [(9, 2), (61, 2), (9, 500), (29, 80), (30, 80), (31, 80), (60, 24), (61, 24)])
+def test_fused_forward_at_the_edges_of_its_tiles(S, grid, B):
+    """The fused forward's tiles are 8 x 14 pixels, or 8 x 30 read as pixel pairs
+    when there are more than six small ones per SM: odd widths (a padded row)
+    and widths at and beside a multiple of 30, few images and many, against the
+    layer-by-layer kernels with the bars of the comparison above."""
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((B, grid, grid, 2)).astype(np.float32)
+    with S.ClosureNet(grid, max_batch=B, seed=3) as net:
+        net.set_scales([1.0, 1.0, 1.0])
+        yf = net.forward(x)
+        net.set_fused(False)
+        yl = net.forward(x)
+    assert _rel(yf, yl) < 2e-3
+    assert np.abs(yf - yl).max() / np.sqrt(np.mean(yl.astype(np.float64) ** 2)) < 2e-2
