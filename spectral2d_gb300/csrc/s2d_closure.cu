@@ -1446,8 +1446,8 @@ cudaError_t launch_wgrad(const __nv_bfloat16* dz, const __nv_bfloat16* in, float
     if (e != cudaSuccess) return e;
     const long ntiles = (long)((Wd + kConvTX - 1) / kConvTX) * ((H + kConvTY - 1) / kConvTY) * B;
     *nblk = (int)std::max<long>(1, std::min<long>(ntiles, grid));
-    return launch_k(k_wgrad_tc<CI, CO>, *nblk, WgTile<CI, CO>::COPY + 32, WgTile<CI, CO>::SMEM, st, false, md, in, part, B, H, Wd,
-                    err);
+    using WT = WgTile<CI, CO>;
+    return launch_k(k_wgrad_tc<CI, CO>, *nblk, WT::COPY + 32, WT::SMEM, st, false, md, in, part, B, H, Wd, err);
 }
 
 // out[i] = sum_b part[b * n + i], b in order; 16 loads in flight per thread,

@@ -32,14 +32,14 @@
 namespace s2d {
 
 // ------------------------------------------------------------------------
-// K1, K2, K3 of one simulation: one tile per CTA (bodies in s2d_step.cuh).
-// K1, K2 and the split K3 come in register budgets B, chosen from the CTA
-// size by budget<T>():
+// K1, K2, K3 of one simulation: one tile per CTA (bodies in s2d_fxstep.cuh and
+// s2d_f32step.cuh for direct plans, s2d_step.cuh for the others).  Register
+// budgets B, chosen at the launches from the CTA size:
 //   B = 1: CTAs of at most 256 threads, FP64 three per SM (80 registers: a
 //          third CTA fills the barrier phases of the other two), FP32 four
 //          (64 registers);
-//   B = 2: FP32 CTAs of at most 512 threads (M = 6144), two per SM (64
-//          registers);
+//   B = 3: CTAs of at most 384 threads, two per SM;
+//   B = 2: CTAs of at most 512 threads (M = 6144), two per SM (64 registers);
 //   B = 0: one CTA of up to 512 threads per SM.
 // (Wider FP32 column tiles -- 2 or 4 columns per CTA of 512 or 1024 threads,
 // so that the half-spectral rows are written and gathered a sector at a
@@ -49,10 +49,6 @@ template <int B>
 constexpr int kMaxThreads = B == 1 ? 256 : (B == 3 ? 384 : 512);
 template <typename T, int B>
 constexpr int kMinBlocks = B == 1 ? (sizeof(T) == 8 ? 3 : 4) : (B >= 2 ? 2 : 1);
-template <typename T>
-int budget(int threads) {
-    return threads <= 256 ? 1 : (sizeof(T) == 4 ? 2 : 0);
-}
 
 template <typename T, int B>
 __global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<T, B>)) k_yinv(Dims d, const typename Vec<T>::t* __restrict__ S,
@@ -126,7 +122,7 @@ __global__ void __launch_bounds__(256) k_stage(Dims d, const typename Vec<T>::t*
 // ---- FP64, direct plans (s2d_fxstep.cuh) ---------------------------------
 // E elements per thread: 12, or 4 for small grids.  CTAs of at most 256
 // threads: three per SM (B = 1, 80 registers); up to 384: two (B = 3, 80; one
-// at 128 took 5.77 against 5.50 ms of the 3072^2 step); up to 512: K1 two
+// at 128: the 3072^2 step 5.77 -> 5.50 ms, 4.84 with the results' conversion); up to 512: K1 two
 // (B = 2, 64), whose loads and stores gain more than its spills cost (4096^2
 // 2.37 -> 2.31 ms), K2 and K3 one (B = 0, 128; two: 4.5 -> 5.0, 2.8 -> 3.3 ms).
 template <int E, int B>
