@@ -249,7 +249,8 @@ HostArray host_array(const s2d_handle* h, const double* p, bool write) {
     HostArray a;
     a.host = const_cast<double*>(p);
     if (!p || h->io_copy_only) return a;
-    a.dev = (double*)device_view(h->device, h->pageable_direct, p, h->ref_bytes, write, &a.pageable);
+    a.dev = (double*)device_view(h->device, h->pageable_direct, p, h->ref_bytes, sizeof(double), write,
+                                 &a.pageable);
     return a;
 }
 
@@ -396,8 +397,10 @@ int spectrum_impl(s2d_handle* h, std::vector<double>& Ek) {
 
 }  // namespace
 
-void* s2d::device_view(int device, bool pageable, const void* p, size_t n, bool write, bool* through_tables) {
+void* s2d::device_view(int device, bool pageable, const void* p, size_t n, size_t align, bool write,
+                       bool* through_tables) {
     *through_tables = false;
+    if ((uintptr_t)p % align) return nullptr;   // (a device address has the same offset in its page)
     void* q = const_cast<void*>(p);
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {

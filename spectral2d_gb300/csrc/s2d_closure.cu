@@ -2224,18 +2224,19 @@ uint64_t mix64(uint64_t x) {
 int upload_host_batch(s2d_cnn* c, const float* x, const float* target, int B) {
     const long P = (long)B * c->H * c->Wd;
     bool tables;
-    const float* xd = (const float*)device_view(c->device, c->pageable_direct, x, 2 * P * sizeof(float), false, &tables);
+    const float* xd = (const float*)device_view(c->device, c->pageable_direct, x, 2 * P * sizeof(float),
+                                                sizeof(float2), false, &tables);
     const float* td = target ? (const float*)device_view(c->device, c->pageable_direct, target, P * sizeof(float),
-                                                         false, &tables)
+                                                         sizeof(float), false, &tables)
                              : nullptr;
     if ((!xd || (target && !td)) && !c->stage)
         C_CUDA(cudaMalloc(&c->stage, 3 * (size_t)c->maxB * c->H * c->Wd * sizeof(float)));
     if (!xd) {
-        C_CUDA(cudaMemcpyAsync(c->stage, x, 2 * P * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+        C_CUDA(cudaMemcpyAsync(c->stage, x, 2 * P * sizeof(float), cudaMemcpyDefault, c->stream));
         xd = c->stage;
     }
     if (target && !td) {
-        C_CUDA(cudaMemcpyAsync(c->stage + 2 * P, target, P * sizeof(float), cudaMemcpyHostToDevice, c->stream));
+        C_CUDA(cudaMemcpyAsync(c->stage + 2 * P, target, P * sizeof(float), cudaMemcpyDefault, c->stream));
         td = c->stage + 2 * P;
     }
     k_pack_pairs<<<nblocks(P, 256), 256, 0, c->stream>>>((const float2*)xd, td, P, (float)(1.0 / c->scale[0]),
@@ -2644,11 +2645,12 @@ S2D_API int s2d_cnn_forward_host(s2d_cnn* c, const float* x, int32_t B, float* y
     if (r != S2D_OK) return r;
     const long P = (long)B * c->H * c->Wd;
     bool tables;
-    float* yd = (float*)device_view(c->device, c->pageable_direct, y, P * sizeof(float), true, &tables);
+    float* yd = (float*)device_view(c->device, c->pageable_direct, y, P * sizeof(float), sizeof(float), true,
+                                   &tables);
     float* dst = yd ? yd : c->tgt;   // the targets are unused here
     k_scale_out<<<nblocks(P, 256), 256, 0, c->stream>>>(c->Y, P, c->scale[2], dst);
     C_CUDA(cudaGetLastError());
-    if (!yd) C_CUDA(cudaMemcpyAsync(y, dst, P * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
+    if (!yd) C_CUDA(cudaMemcpyAsync(y, dst, P * sizeof(float), cudaMemcpyDefault, c->stream));
     C_CUDA(cudaStreamSynchronize(c->stream));
     return s2d_cnn_status(c);
 }

@@ -334,8 +334,10 @@ int create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handle** o
 // The address at which the device reaches n bytes of a caller's array in
 // place: page-locked or device memory, or (pageable) ordinary host memory
 // through the host page tables where its pages are resident; writable arrays
-// whose pages are not are populated first.  Null: copy instead.
-void* device_view(int device, bool pageable, const void* p, size_t n, bool write, bool* through_tables);
+// whose pages are not are populated first.  Null: copy instead; so for an
+// address that is no multiple of align, the size of what the kernels load and
+// store there.
+void* device_view(int device, bool pageable, const void* p, size_t n, size_t align, bool write, bool* through_tables);
 
 // Shared-memory attribute setup (called once per process and device).
 cudaError_t configure_kernels(int max_smem_optin);

@@ -1,0 +1,49 @@
+"""GPU tests of the caller's arrays at addresses that the kernels' loads and
+stores do not take in place: such arrays go through staging copies, with the
+same results as aligned ones."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def S(built_lib):
+    import spectral2d_gb300
+    return spectral2d_gb300
+
+
+def _at(values, offset, mem="pageable"):
+    """A copy of the array that starts `offset` bytes past a 64-byte boundary."""
+    from spectral2d_gb300.solver import pinned_array
+    n = values.nbytes + 128
+    raw = pinned_array(n, np.uint8) if mem == "pinned" else np.zeros(n, dtype=np.uint8)
+    at = -raw.ctypes.data % 64 + offset
+    a = raw[at:at + values.nbytes].view(values.dtype).reshape(values.shape)
+    a[...] = values
+    assert a.ctypes.data % 64 == offset and a.flags.c_contiguous
+    return a
+
+
+@pytest.mark.parametrize("mem", ["pageable", "pinned"])
+@pytest.mark.parametrize("offset", [2, 4, 8, 12])
+def test_closure_batches_at_any_address(S, offset, mem):
+    """(omega, psi) pairs are loaded 8 bytes at a time; a float array may start
+    at any multiple of 4, or (packed buffers) anywhere."""
+    from spectral2d_gb300 import _lib as L
+    from spectral2d_gb300.solver import _fptr
+    rng = np.random.default_rng(offset)
+    x = _at(rng.standard_normal((3, 24, 24, 2)).astype(np.float32), 0)
+    t = _at(rng.standard_normal((3, 24, 24)).astype(np.float32), 0)
+    with S.ClosureNet(24, max_batch=4, seed=1) as net:
+        y = net.forward(x)
+        loss, g = net.grad(x, t)
+        xo, to = _at(x, offset, mem), _at(t, offset, mem)
+        assert np.array_equal(net.forward(xo), y)
+        for a, b in ((xo, to), (xo, t), (x, to)):
+            lo, go = net.grad(a, b)
+            assert lo == loss and np.array_equal(go, g)
+        yo = _at(np.zeros_like(y), offset, mem)
+        L.check(net._L.s2d_cnn_forward_host(net._c, _fptr(x), 3, _fptr(yo)))
+        assert np.array_equal(yo, y)
