@@ -208,7 +208,8 @@ int ensure_ref_stage(s2d_handle* h) {
 // A host array of a host-array call, as the kernels reach it: in place
 // through a device-usable address (page-locked memory; pageable memory where
 // the device reads the host page tables, as on Grace; device memory), or,
-// with dev null, through the staging arrays and copies.
+// with dev null, through the staging arrays and copies.  The kernels move whole
+// complex numbers, so an array that is not 16-byte aligned is staged too.
 struct HostArray {
     double* host = nullptr;
     double* dev = nullptr;
@@ -249,7 +250,7 @@ HostArray host_array(const s2d_handle* h, const double* p, bool write) {
     HostArray a;
     a.host = const_cast<double*>(p);
     if (!p || h->io_copy_only) return a;
-    a.dev = (double*)device_view(h->device, h->pageable_direct, p, h->ref_bytes, sizeof(double), write,
+    a.dev = (double*)device_view(h->device, h->pageable_direct, p, h->ref_bytes, sizeof(double2), write,
                                  &a.pageable);
     return a;
 }

@@ -47,3 +47,42 @@ def test_closure_batches_at_any_address(S, offset, mem):
         yo = _at(np.zeros_like(y), offset, mem)
         L.check(net._L.s2d_cnn_forward_host(net._c, _fptr(x), 3, _fptr(yo)))
         assert np.array_equal(yo, y)
+
+
+@pytest.mark.parametrize("mem", ["pageable", "pinned", "fresh"])
+@pytest.mark.parametrize("n", [24, 96])
+def test_state_arrays_at_half_an_element(S, n, mem):
+    """The kernels move complex numbers 16 bytes at a time; an array of doubles
+    may start 8 bytes off, its pages touched already or not."""
+    import oracle as O
+    from spectral2d_gb300 import _lib as L
+    from spectral2d_gb300.solver import _dptr
+    w = O.random_state(O.get_grid_size(n, n), 5, decay=0.1)
+
+    def buf(values=None):
+        if mem == "fresh" and values is None:
+            raw = np.zeros(2 * w.size + 8)   # pages not touched yet
+            at = (-raw.ctypes.data % 16) // 8 + 1
+            a = raw[at:at + 2 * w.size].view(np.complex128).reshape(w.shape)
+        else:
+            a = _at(np.full_like(w, np.nan) if values is None else values, 8, "pinned" if mem == "pinned" else "pageable")
+        assert a.ctypes.data % 16 == 8
+        return a
+
+    shape = w.shape[::-1]
+    with S.Spectral2D(n, nu=0.01) as r:
+        r.set_state(w)
+        dW = r.compute_rhs()
+        r.integrate_one_step(1e-3)
+        w1, p1 = r.get_state()
+    with S.Spectral2D(n, nu=0.01) as s:
+        s.set_state(buf(w))
+        d = buf()
+        L.check(s._L.s2d_compute_rhs(s._h, _dptr(d.view(np.float64)), *shape))
+        gw, gp = buf(w), buf()
+        s.integrate_one_step_host(gw, 1e-3, gp, inplace=True)
+        hw, hp = buf(), np.full_like(w, np.nan)   # one staged, one in place
+        L.check(s._L.s2d_get_state(s._h, _dptr(hw.view(np.float64)), _dptr(hp.view(np.float64)), *shape))
+    assert np.array_equal(d, dW)
+    for a, b in ((gw, w1), (gp, p1), (hw, w1), (hp, p1)):
+        assert np.array_equal(a, b)
