@@ -25,6 +25,7 @@
 #include "s2d.h"
 #include "s2d_internal.h"
 #include "s2d_f32step.cuh"
+#include "s2d_frame.cuh"
 #include "s2d_step.cuh"
 
 #include <cuda.h>
@@ -686,7 +687,6 @@ cudaError_t launch_conv(const __nv_bfloat16* in, const __nv_bfloat16* W, const f
 // Every wait is bounded: a wait that runs out sets bit 4 of *err and
 // the abort flag, the CTA skips the rest (after bounded waits for its copies
 // and MMAs in flight) and frees its tensor memory.
-__host__ __device__ inline int net_pitch(int Wd) { return (Wd + 3) & ~1; }   // pixels of a framed row, even
 constexpr int kNetGroups = 2;                    // epilogue groups of 8 warps (tile i: group i % 2)
 // Tile i uses box slot i % 4 and accumulator i % (4 / P); one commit per tile (mmad of
 // the slot) tells the epilogue the accumulator is ready and the producer the
@@ -1100,8 +1100,7 @@ __global__ void k_frame16(const __nv_bfloat16* __restrict__ x, int B, int H, int
         p /= fw;
         const int fy = (int)(p % fh);
         const long b = p / fh;
-        const int yy = fy == 0 ? H - 1 : (fy == H + 1 ? 0 : fy - 1);
-        const int xx = fx == 0 ? Wd - 1 : (fx == Wd + 1 ? 0 : fx - 1);
+        const int yy = net_frame_source(fy, H), xx = net_frame_source(fx, Wd);
         reinterpret_cast<uint4*>(xf)[i] =
             reinterpret_cast<const uint4*>(x)[((b * H + yy) * Wd + xx) * 2 + q];
     }
