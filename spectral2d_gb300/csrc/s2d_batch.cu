@@ -22,6 +22,7 @@
 // The tuner (s2d_batch_tune) times candidate tile schedules -- threads per
 // CTA (and so transforms per tile) and CTAs per SM -- on the actual ensemble
 // and keeps the fastest; the state is restored afterwards.
+#define S2D_FX_GROUPS 256   // 512 threads on transforms of 24 elements
 #include "s2d.h"
 #include "s2d_internal.h"
 #include "s2d_f32step.cuh"
@@ -371,7 +372,7 @@ S2D_API int s2d_batch_create(int32_t nruns, const s2d_config* cfgs, s2d_batch** 
     cudaDeviceProp prop{};
     if (cudaGetDeviceProperties(&prop, b->device) != cudaSuccess) return bail(berr(S2D_ERR_CUDA, "device query"));
     b->sms = prop.multiProcessorCount;
-    b->max_smem = (int)prop.sharedMemPerBlockOptin - kStaticSmem;
+    b->max_smem = (int)prop.sharedMemPerBlockOptin - kStaticSmem - 32 * S2D_FX_GROUPS;
     for (int i = 0; i < nruns; ++i) {
         s2d_handle* h = nullptr;
         const int r = create_handle(&cfgs[i], b->stream, &h);

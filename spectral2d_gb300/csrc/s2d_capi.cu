@@ -109,7 +109,10 @@ int pick_launch(const s2d_handle* h, int threads_per_group, size_t bytes_per_gro
     const int gmax = std::max(1, target_threads / threads_per_group);
     const int gmin = std::max(1, (32 + threads_per_group - 1) / threads_per_group);
     const long gfill = (items + 2L * h->sms - 1) / (2L * h->sms);
-    int G = (int)std::max<long>(gmin, std::min<long>(gmax, gfill));
+    // (32 groups of a one-thread transform fill a warp; the forward y-pass runs
+    // up to two transforms per group at a time)
+    static_assert(2 * 32 <= kFxGroups);
+    int G = (int)std::max<long>(gmin, std::min<long>({gmax, gfill, 32}));
     while (G > 1 && (G * threads_per_group > 512 || G * bytes_per_group > cap_pair)) --G;
     L->G = G;
     L->threads = G * threads_per_group;

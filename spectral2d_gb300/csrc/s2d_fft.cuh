@@ -373,13 +373,35 @@ __device__ __forceinline__ void fft_pass2_fma(VT* buf, int M, int Ns, unsigned m
 // (E = 12 or 4 elements per thread); the forward transforms of direct plans
 // (Dims::direct) run the radices in reverse order.
 
-// Reduction words of the CTA's transforms, zeroed by their first users: the
-// largest high word of the input, the sum of its magnitudes, and the same of
-// a second transform of the row (x-pass).
-constexpr int kFxWords = 1024;
+// Words of the CTA's transforms, eight each, set by their first users: the
+// largest high word of the input, the sum of its magnitudes, the same of a
+// second transform of the row, and a constant (re, im) that is kept out of the
+// transform.  S2D_FX_GROUPS transforms per CTA at most: kFxGroups in the single
+// runs' launches, 256 in the batch's.  (8 KB in all of them left the 2048^2
+// kernels less L1 beside their three CTAs' shared memory: K3 631 -> 660 us per
+// step.)
+#ifndef S2D_FX_GROUPS
+#define S2D_FX_GROUPS kFxGroups
+#endif
 __device__ __forceinline__ int* fx_words() {
-    __shared__ int w[kFxWords];
+    __shared__ __align__(16) int w[8 * S2D_FX_GROUPS];
     return w;
+}
+// Whether element 0 of an inverse transform of M elements, of magnitude m0, is
+// so large beside the rest, of magnitude mr (both fx_magnitude), that the
+// common exponent takes more bits from the rest than FP64 would.  It is then
+// kept out of the fixed point and added in FP64: it enters every result alike,
+// as in an FP64 transform, whose butterflies never twiddle it, so that its real
+// part (the mean of u) takes no bits from the other results' imaginary parts
+// (v).  With it always in, the tendency of ky = 0 of a perturbation 1e-6 of a
+// flow that depends on y alone had errors of 3e-11 (64^2), in FP64 3e-15.
+// The line: one large element alone leaves an error of about 0.6 sqrt(M) 2^-60
+// of it, 2.9e-17 for M = 3072; the rest, smaller by up to 8 (16 for M <= 1024),
+// keeps 2e-16 of its norm, an FP64 transform's.  Kept out where two numbers
+// differ by a factor of two already, some rows of ordinary turbulence are, which
+// then read their spectra again (96^2: 63.5 -> 65.5 us per step).
+__device__ __forceinline__ bool fx_constant_out(int m0, int mr, int M) {
+    return (m0 >> 20) > (mr >> 20) + (M <= 1024 ? 3 : 2);
 }
 // Maximum or sum over a transform into a zeroed word.  whole: the transform
 // owns whole warps (32 divides T).
@@ -428,17 +450,38 @@ __device__ __forceinline__ int swz(int i) { return i ^ ((i >> 3) & 3) ^ ((i >> 2
 // base of the four elements 4 j .. 4 j + 3 (element r at base ^ r)
 __device__ __forceinline__ int swz4(int j, bool on) { return on ? swz(4 * j) : 4 * j; }
 
-// The twiddled inputs of butterfly position k: r bits shifted out on the way.
+// The twiddled inputs of a butterfly, r bits shifted out on the way: by the R - 1
+// factors w, or by those of position k of the table, read ahead of the first
+// product or one by one.  Ahead, the direct kernels need fewer registers (80 at
+// three CTAs per SM: 2048^2 K1 417 -> 392, K2 874 -> 833, K3 629 -> 610 us per
+// step); fx_run only waits for them at once (512^2 conservative 291 -> 295).
+__device__ __forceinline__ FxTw fx_tw(const FxTw* __restrict__ tab) {
+    const int4 w = __ldg(reinterpret_cast<const int4*>(tab));
+    return FxTw{w.x, w.y, w.z, w.w};
+}
 template <int R, bool INV>
-__device__ __forceinline__ void fx_twiddle(fx2* v, const FxTw* __restrict__ tab, int Ns, int k, int rsh) {
+__device__ __forceinline__ void fx_twiddle_by(fx2* v, const FxTw* w, int rsh) {
     if (rsh) {
         v[0].x = fx_round(v[0].x, rsh);
         v[0].y = fx_round(v[0].y, rsh);
     }
 #pragma unroll
-    for (int r = 1; r < R; ++r) {
-        const int4 w = __ldg(reinterpret_cast<const int4*>(tab + (r - 1) * Ns + k));
-        v[r] = fx_cmul<INV>(v[r], FxTw{w.x, w.y, w.z, w.w}, rsh);
+    for (int r = 1; r < R; ++r) v[r] = fx_cmul<INV>(v[r], w[r - 1], rsh);
+}
+template <int R, bool INV, bool AHEAD>
+__device__ __forceinline__ void fx_twiddle(fx2* v, const FxTw* __restrict__ tab, int Ns, int k, int rsh) {
+    if constexpr (AHEAD) {
+        FxTw w[R - 1];
+#pragma unroll
+        for (int r = 1; r < R; ++r) w[r - 1] = fx_tw(tab + (r - 1) * Ns + k);
+        fx_twiddle_by<R, INV>(v, w, rsh);
+    } else {
+        if (rsh) {
+            v[0].x = fx_round(v[0].x, rsh);
+            v[0].y = fx_round(v[0].y, rsh);
+        }
+#pragma unroll
+        for (int r = 1; r < R; ++r) v[r] = fx_cmul<INV>(v[r], fx_tw(tab + (r - 1) * Ns + k), rsh);
     }
 }
 template <int R, bool INV>
@@ -449,11 +492,13 @@ __device__ __forceinline__ void fx_butterfly(fx2* v) {
 }
 
 // One pass after the first, in place (all loads, barrier, all stores,
-// barrier).  LAST: results rounded to FP64, eb their exponent base (fx_to).
+// barrier).  LAST: results rounded to FP64, eb their exponent base (fx_to), *c a
+// constant to add (or null).
 // lsw: the permutation of the lane for the loads (swz), or the lane.
-template <int E, int R, bool INV, bool LAST = false>
+template <int E, int R, bool INV, bool LAST = false, bool AHEAD = false>
 __device__ __forceinline__ void fx_pass(longlong2* buf, int M, int Ns, unsigned mg, int lane, int T,
-                                        const FxTw* __restrict__ tab, int rsh, int lsw, int eb = 0) {
+                                        const FxTw* __restrict__ tab, int rsh, int lsw, int eb = 0,
+                                        const double2* c = nullptr) {
     constexpr int NB = kFxNB<E, R>;
     fx2 v[NB][R];
     const int stride = M / R;
@@ -471,13 +516,14 @@ __device__ __forceinline__ void fx_pass(longlong2* buf, int M, int Ns, unsigned 
         const int j = lane + b * T;
         if (!fx_on<E, R>(j, M)) continue;
         const int k = mod(j);
-        fx_twiddle<R, INV>(v[b], tab, Ns, k, rsh);
+        fx_twiddle<R, INV, AHEAD>(v[b], tab, Ns, k, rsh);
         fx_butterfly<R, INV>(v[b]);
         const int base = (j - k) * R + k;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if constexpr (LAST) {
-                const double2 z = fx_to(v[b][r], eb);
+                double2 z = fx_to(v[b][r], eb);
+                if (INV && c) z = make_double2(z.x + c->x, z.y + c->y);
                 buf[base + r * Ns] = make_longlong2(__double_as_longlong(z.x), __double_as_longlong(z.y));
             } else {
                 fx_st(buf, base + r * Ns, v[b][r]);
@@ -499,9 +545,9 @@ __device__ __forceinline__ void fx_middle(longlong2* buf, const Dims& d, int lan
         const FxTw* tp = tab + (INV ? d.twoff[p] : d.twofff[p]);
         const int tn = max(t, fx_shift_total(Ns * R, per, sum, by_limit));
         const int lsw = !INV && p == 1 && swz_on(d, T) ? swz(lane) : lane;
-        if (R == 4) fx_pass<E, 4, INV>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lsw);
-        else if (R == 2) fx_pass<E, 2, INV>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lane);
-        else fx_pass<E, 3, INV>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lane);
+        if (R == 4) fx_pass<E, 4, INV, false, true>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lsw);
+        else if (R == 2) fx_pass<E, 2, INV, false, true>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lane);
+        else fx_pass<E, 3, INV, false, true>(buf, d.M, Ns, mg, lane, T, tp, tn - t, lane);
         t = tn;
         Ns *= R;
     }
@@ -510,13 +556,15 @@ __device__ __forceinline__ void fx_middle(longlong2* buf, const Dims& d, int lan
 // ---- the general FP64 transform, FP64 in and out (fft_run) -----------------
 // First pass: the E elements of the thread from FP64, their common exponent
 // emax, the sum of magnitudes, a radix-R DFT without twiddles.  PRUNE: radix 3
-// with the middle input zero but for j = 0 (see fft_pass3_midzero).
+// with the middle input zero but for j = 0 (see fft_pass3_midzero).  out (INV):
+// element 0 was kept out (fx_constant_out) and is in words + 4.
 template <int E, int R, bool INV, bool PRUNE>
-__device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg, int n0, int* words) {
+__device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg, int n0, int* words, bool& out) {
     constexpr int NB = kFxNB<E, R>;
     double2 z[NB][R];
     const int stride = M / R;
     int mx = 0;
+    const int m0 = INV ? fx_magnitude(reinterpret_cast<const double2*>(buf)[0]) : 0;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * Tg;
@@ -525,13 +573,18 @@ __device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg,
         for (int r = 0; r < R; ++r) {
             if (PRUNE && r == 1 && (b > 0 || j > 0)) continue;
             z[b][r] = reinterpret_cast<const double2*>(buf)[j + r * stride];
-            mx = max(mx, fx_magnitude(z[b][r]));
+            if (!INV || r || b || lane) mx = max(mx, fx_magnitude(z[b][r]));
         }
     }
     const bool whole = (Tg & 31) == 0;
     fx_reduce_max(&words[0], mx, lane, whole);
     __syncthreads();
-    const int emax = words[0] >> 20;
+    out = INV && fx_constant_out(m0, words[0], M);
+    const int emax = (out ? words[0] : max(m0, words[0])) >> 20;
+    if (out && lane == 0) {
+        *reinterpret_cast<double2*>(words + 4) = z[0][0];
+        z[0][0] = make_double2(0.0, 0.0);
+    }
     unsigned sum = 0;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
@@ -553,29 +606,30 @@ __device__ __forceinline__ int fx_first(longlong2* buf, int M, int lane, int Tg,
 #pragma unroll
         for (int r = 0; r < R; ++r) fx_st(buf, j * R + r, v[r]);
     }
-    fx_reduce_add(&words[512], sum, lane, whole);
+    fx_reduce_add(&words[1], sum, lane, whole);
     __syncthreads();
     return emax;
 }
 
-// The FP64 transform (see fft_run).  A transform with an infinity or NaN
-// gives NaN throughout.
-template <bool INV, int E>
+// The FP64 transform (see fft_run).  An infinity or NaN reaches every result.
+template <bool INV, int E, bool APART>
 __device__ __forceinline__ void fx_run(longlong2* buf, const Dims& d, int lane, const FxTw* __restrict__ tab) {
-    int* words = fx_words() + ((int)threadIdx.x - lane);
-    if (lane == 0) {
-        words[0] = 0;
-        words[512] = 0;
-    }
+    int* words = fx_words() + 8 * ((int)threadIdx.x / d.Tg);
+    if (lane == 0) words[0] = words[1] = 0;
     __syncthreads();
     const int R0 = d.radix[0];
     const int n0 = R0 == 4 ? 4 : 3;
     int emax;
-    if (INV && R0 == 3 && 3 * d.K == d.M) emax = fx_first<E, 3, INV, INV>(buf, d.M, lane, d.Tg, n0, words);
-    else if (R0 == 3) emax = fx_first<E, 3, INV, false>(buf, d.M, lane, d.Tg, n0, words);
-    else if (R0 == 4) emax = fx_first<E, 4, INV, false>(buf, d.M, lane, d.Tg, n0, words);
-    else emax = fx_first<E, 2, INV, false>(buf, d.M, lane, d.Tg, n0, words);
-    const unsigned sum = (unsigned)words[512];
+    bool out;
+    if (INV && R0 == 3 && 3 * d.K == d.M) emax = fx_first<E, 3, INV, INV>(buf, d.M, lane, d.Tg, n0, words, out);
+    else if (R0 == 3) emax = fx_first<E, 3, INV, false>(buf, d.M, lane, d.Tg, n0, words, out);
+    else if (R0 == 4) emax = fx_first<E, 4, INV, false>(buf, d.M, lane, d.Tg, n0, words, out);
+    else emax = fx_first<E, 2, INV, false>(buf, d.M, lane, d.Tg, n0, words, out);
+    const unsigned sum = (unsigned)words[1];
+    if (INV && APART && lane == 0) {
+        words[3] = out;
+        if (!out) *reinterpret_cast<double2*>(words + 4) = make_double2(0.0, 0.0);
+    }
     const float per = fx_per(n0);
     int Ns = R0, t = 0;
     for (int p = 1; p < d.npass; ++p) {
@@ -591,12 +645,25 @@ __device__ __forceinline__ void fx_run(longlong2* buf, const Dims& d, int lane, 
             else fx_pass<E, 3, INV>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane);
         } else {
             const int eb = fx_exponent_base(emax, n0, t);
-            if (R == 4) fx_pass<E, 4, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb);
-            else if (R == 2) fx_pass<E, 2, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb);
-            else fx_pass<E, 3, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb);
+            const double2* c = INV && !APART && out ? reinterpret_cast<const double2*>(words + 4) : nullptr;
+            if (R == 4) fx_pass<E, 4, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb, c);
+            else if (R == 2) fx_pass<E, 2, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb, c);
+            else fx_pass<E, 3, INV, true>(buf, d.M, Ns, mg, lane, d.Tg, tp, rsh, lane, eb, c);
         }
         Ns *= R;
     }
+}
+
+// The constant that an FP64 inverse transform with APART left out of its
+// results (zero and false if none), from its end to the next one's start; g:
+// the transform's group of the CTA.
+struct FxMean {
+    double2 m;
+    bool out;
+};
+__device__ __forceinline__ FxMean fx_mean(int g) {
+    const int* words = fx_words() + 8 * g;
+    return FxMean{*reinterpret_cast<const double2*>(words + 4), words[3] != 0};
 }
 
 // FP32: passes [p0, p1) of the plan over the transform in buf.
@@ -633,11 +700,12 @@ __device__ __forceinline__ void f32_passes(float2* buf, const Dims& d, int lane,
 // (Dims::twoff, tab_bytes).  Inverse transforms of truncated spectra (input
 // zero for K < n < M - K, K = M/3: the inverse transforms of this library)
 // take the pruned first radix-3 pass.  E elements per thread (d.Tg = M / E).
-template <bool INV, int E = kElemsPerThread, typename VT>
+// APART: an inverse transform may leave its element 0 to the caller (fx_mean).
+template <bool INV, int E = kElemsPerThread, bool APART = false, typename VT>
 __device__ __forceinline__ void fft_run(VT* buf, const Dims& d, int lane, const VT* __restrict__ tw) {
     using T = decltype(buf[0].x);
     if constexpr (sizeof(T) == 8) {
-        fx_run<INV, E>(reinterpret_cast<longlong2*>(buf), d, lane, reinterpret_cast<const FxTw*>(tw));
+        fx_run<INV, E, APART>(reinterpret_cast<longlong2*>(buf), d, lane, reinterpret_cast<const FxTw*>(tw));
     } else {
         __syncthreads();
         f32_passes<E, INV>(buf, d, lane, tw, 0, d.npass);

@@ -6,6 +6,8 @@
 // p passes exchanges its elements p - 1 times through shared memory.
 #pragma once
 
+#include <type_traits>
+
 #include "s2d_step.cuh"
 
 namespace s2d {
@@ -34,7 +36,7 @@ __device__ __forceinline__ void fx_yinv_body(const Dims& d, const double2* __res
     }
     if (op == OP_TU || op == OP_TV) rk2 = tab;   // the factor table takes the 1/k^2 table's place
     longlong2* buf = reinterpret_cast<longlong2*>(bufs + (size_t)g * M);
-    int* words = fx_words() + 4 * g;
+    int* words = fx_words() + 8 * g;
     if (lane == 0) words[0] = words[1] = 0;
     const double2* col = S + (size_t)(active ? kx : 0) * d.ldS;
     const double* rcol = rk2 + (size_t)(active ? kx : 0) * d.ldS;
@@ -108,7 +110,7 @@ __device__ __forceinline__ void fx_yinv_body(const Dims& d, const double2* __res
         fx2 v[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) v[r] = fx_ld(buf, j + r * (M / 4));
-        fx_twiddle<4, true>(v, tp, M / 4, j, tn - t);
+        fx_twiddle<4, true, true>(v, tp, M / 4, j, tn - t);
         fx_bf4<true>(v);
         if (active) {
 #pragma unroll
@@ -127,6 +129,11 @@ __device__ __forceinline__ void fx_yinv_body(const Dims& d, const double2* __res
 // last one belong to the same two entries of the half spectra, so that the
 // Hermitian extension and the split stay in registers.  q = 0 pairs 0 with
 // K / 2 and takes z(K), P(K) besides.
+// Where the row's means (kx = 0) would take bits from the rest
+// (fx_constant_out) they are left out of the transforms, and the products'
+// parts that are linear in the rest are added in FP64 (linear_part_bas): at
+// the end, in a copy of the last pass, so that other rows' carries no more
+// than a branch (in one copy: 2048^2 K2 833 -> 880 us per step).
 // scale: factor of the results (1 when u and v are prescaled).
 template <int E>
 __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double2* Iv, const FxTw* __restrict__ tw,
@@ -139,10 +146,11 @@ __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double
     const int y = blk * G + g;
     const bool active = y < d.rows && g < G;
     longlong2* buf = reinterpret_cast<longlong2*>(bufs + (size_t)g * M);
-    int* words = fx_words() + 4 * g;
-    if (lane == 0) words[0] = words[1] = words[2] = words[3] = 0;
+    int* words = fx_words() + 8 * g;
+    if (lane == 0) *reinterpret_cast<int4*>(words) = make_int4(0, 0, 0, 0);
     double2* urow = Iu + (size_t)(active ? y : 0) * d.ldI;
     double2* vrow = Iv + (size_t)(active ? y : 0) * d.ldI;
+    double2* means = reinterpret_cast<double2*>(words + 4);
     const bool whole = (T & 31) == 0;
 
     // ---- inverse, first pass
@@ -165,14 +173,20 @@ __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double
         vm = __ldcg(&vrow[K]);
         ua[0].y = va[0].y = 0.0;   // kx = 0 contributes its real parts only
     }
+    if (lane == 0) *means = make_double2(ua[0].x, va[0].x);
 #pragma unroll
-    for (int p = 0; p < NP; ++p)
-        mx = max(mx, max(max(fx_magnitude(ua[p]), fx_magnitude(va[p])), max(fx_magnitude(ub[p]), fx_magnitude(vb[p]))));
+    for (int p = 0; p < NP; ++p) {
+        mx = max(mx, max(fx_magnitude(ub[p]), fx_magnitude(vb[p])));
+        if (p || lane) mx = max(mx, max(fx_magnitude(ua[p]), fx_magnitude(va[p])));
+    }
     mx = max(mx, max(fx_magnitude(um), fx_magnitude(vm)));
     __syncthreads();
     fx_reduce_max(&words[0], mx, lane, whole);
     __syncthreads();
-    const int emax = words[0] >> 20;
+    const int m0 = fx_magnitude(*means), mr = words[0];
+    const bool out = fx_constant_out(m0, mr, M);   // (the means are looked at apart)
+    const int emax = (out ? mr : max(m0, mr)) >> 20;
+    if (out && lane == 0) ua[0].x = va[0].x = 0.0;
     unsigned sum = 0;
     // components below 2^59 (n0 = 4), so that those of u + i v are below 2^60
     auto zp = [](fx2 a, fx2 b) { return fx2{a.x - b.y, a.y + b.x}; };    // z(k)
@@ -221,7 +235,7 @@ __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double
         const int j = lane + b * T;
 #pragma unroll
         for (int r = 0; r < 4; ++r) z[b][r] = fx_ld(buf, j + r * (M / 4));
-        fx_twiddle<4, true>(z[b], tw + d.twoff[d.npass - 1], M / 4, j, tn - t);
+        fx_twiddle<4, true, true>(z[b], tw + d.twoff[d.npass - 1], M / 4, j, tn - t);
         fx_bf4<true>(z[b]);
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -272,38 +286,58 @@ __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double
     const int tf = max(t, fx_shift_total(M, per, sum, 2.0f * kFxByLimit));
     if (ebp < 1 << 16) ebp += tf;
     const FxTw* tp = tw + d.twofff[d.npass - 1];
-    auto put = [&](int k, fx2 p, fx2 c) {   // c = P(M - k)
+    auto put = [&](auto add, int k, fx2 p, fx2 c) {   // c = P(M - k)
         double2 a = fx_to(fx2{p.x + c.x, p.y - c.y}, ebp), b = fx_to(fx2{p.y + c.y, c.x - p.x}, ebp);
         if (scale != 1.0) {
             a = make_double2(a.x * scale, a.y * scale);
             b = make_double2(b.x * scale, b.y * scale);
         }
+        if constexpr (add.value) {   // (this thread alone reads and writes entry k)
+            double2 U = __ldcg(&urow[k]), V = __ldcg(&vrow[k]);
+            linear_part_bas(U, V, *reinterpret_cast<const double2*>(words + 4), 2.0 * M * scale, k == 0);
+            a = make_double2(a.x + U.x, a.y + U.y);
+            b = make_double2(b.x + V.x, b.y + V.y);
+        }
         urow[k] = a;
         vrow[k] = b;
     };
+    // the first butterflies' twiddles, read before the branch so as not to wait
+    // for them behind the last barrier
+    const FxTw t0[2] = {fx_tw(tp + lane), fx_tw(tp + K + lane)};
+    const int l2 = lane ? K - lane : K / 2;
+    const FxTw t1[2] = {fx_tw(tp + l2), fx_tw(tp + K + l2)};
+    auto split = [&](auto add) {
+#pragma unroll(add.value ? 1 : NP)
+        for (int p = 0; p < NP; ++p) {   // (unrolled, the rare form would spill)
+            const int q = lane + p * T;
+            if (E != 12 && q >= K / 2) continue;
+            const int q2 = q ? K - q : K / 2;
+            fx2 v[3], w[3];
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        const int q = lane + p * T;
-        if (E != 12 && q >= K / 2) continue;
-        const int q2 = q ? K - q : K / 2;
-        fx2 v[3], w[3];
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-            v[r] = fx_ld(buf, q + r * K);
-            w[r] = fx_ld(buf, q2 + r * K);
+            for (int r = 0; r < 3; ++r) {
+                v[r] = fx_ld(buf, q + r * K);
+                w[r] = fx_ld(buf, q2 + r * K);
+            }
+            if (p == 0) {
+                fx_twiddle_by<3, false>(v, t0, tf - t);
+                fx_twiddle_by<3, false>(w, t1, tf - t);
+            } else {
+                fx_twiddle<3, false, true>(v, tp, K, q, tf - t);
+                fx_twiddle<3, false, true>(w, tp, K, q2, tf - t);
+            }
+            if (p == 0 && lane == 0) fx_bf3<false>(v);
+            else fx_bf3_02<false>(v);
+            fx_bf3_02<false>(w);
+            if (active) {
+                const bool first = p == 0 && lane == 0;
+                if (first) put(add, K, v[1], v[2]);
+                put(add, q, v[0], first ? v[0] : w[2]);
+                put(add, q2, w[0], first ? w[2] : v[2]);
+            }
         }
-        fx_twiddle<3, false>(v, tp, K, q, tf - t);
-        fx_twiddle<3, false>(w, tp, K, q2, tf - t);
-        if (p == 0 && lane == 0) fx_bf3<false>(v);
-        else fx_bf3_02<false>(v);
-        fx_bf3_02<false>(w);
-        if (active) {
-            const bool first = p == 0 && lane == 0;
-            if (first) put(K, v[1], v[2]);
-            put(q, v[0], first ? v[0] : w[2]);
-            put(q2, w[0], first ? w[2] : v[2]);
-        }
-    }
+    };
+    if (out) split(std::true_type{});
+    else split(std::false_type{});
 }
 
 // K3's transform: column kx of one product, read from the half-spectral rows
@@ -316,7 +350,7 @@ __device__ __forceinline__ void fx_yfwd_column(const Dims& d, const double2* __r
                                                Sink sink) {
     constexpr int NB = kFxNB<E, 4>, N3 = kFxNB<E, 3>;
     const int M = d.M, K = d.K, T = d.Tg;
-    int* words = fx_words() + 4 * g;
+    int* words = fx_words() + 8 * g;
     if (lane == 0) words[0] = words[1] = 0;
     double2 x[NB][4];
     int mx = 0;
@@ -372,7 +406,7 @@ __device__ __forceinline__ void fx_yfwd_column(const Dims& d, const double2* __r
     for (int b = 0; b < N3; ++b) {
         const int j = lane + b * T;
         if (!fx_on<E, 3>(j, M)) continue;
-        fx_twiddle<3, false>(v[b], tp, K, j, tn - t);
+        fx_twiddle<3, false, true>(v[b], tp, K, j, tn - t);
         if (b == 0 && lane == 0) {
             fx_bf3<false>(v[b]);
             sink(K, fx_to(v[b][1], eb));

@@ -23,9 +23,12 @@ namespace s2d {
 
 constexpr int kMaxPasses = 16;
 constexpr int kElemsPerThread = 12;   // FFT elements held per thread per pass
-// shared memory kept for the kernels' static arrays (the FP64 transforms'
-// reduction words, 4 KB, and the reductions of the diagnostics)
+// shared memory kept for the kernels' static arrays (the FP64 transforms' words,
+// 4 KB, and the reductions of the diagnostics)
 constexpr int kStaticSmem = 1024 + 4096;
+// transforms per CTA, at most, in every launch but the batch's (the number of
+// the FP64 transforms' words)
+constexpr int kFxGroups = 128;
 // the FP32 x-pass with register radix-12/16 passes (s2d_xpass32.cuh): row
 // length and its padded shared-memory buffer (elements)
 constexpr int kX32M = 3072;

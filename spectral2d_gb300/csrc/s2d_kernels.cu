@@ -201,6 +201,13 @@ __global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<float, B>))
 // u*w + i v*w, then its spectrum.  On exit rows y of Iu / Iv hold the
 // normalised half spectra of u*w / v*w.
 // ------------------------------------------------------------------------
+__device__ __forceinline__ void extract_pair_rhs(const double2* Z, double2* urow, double2* vrow, const double2* wrow,
+                                                 const Dims& d, int lane, double scale, double2 m, double w0) {
+    extract_pair_add(Z, urow, vrow, d, lane, scale, [&](int k, double2& U, double2& V) {
+        linear_part_rhs(U, V, __ldcg(&wrow[k]), m, w0, 2.0 * d.M * scale, k == 0);
+    });
+}
+
 template <typename T>
 __global__ void __launch_bounds__(512) k_xpass_rhs(Dims d, typename Vec<T>::t* Iu, typename Vec<T>::t* Iv,
                                                     const typename Vec<T>::t* __restrict__ Iw,
@@ -220,7 +227,9 @@ __global__ void __launch_bounds__(512) k_xpass_rhs(Dims d, typename Vec<T>::t* I
     VT* Z = W + d.M;
 
     build_pair(W, Iw + (size_t)y1 * d.ldI, Iw + (size_t)y2 * d.ldI, d, lane, active);
-    fft_run<true>(W, d, lane, tw);
+    fft_run<true, kElemsPerThread, true>(W, d, lane, tw);
+    FxMean wm{};
+    if constexpr (sizeof(T) == 8) wm = fx_mean(g);
 
 #pragma unroll 1
     for (int h = 0; h < 2; ++h) {
@@ -228,14 +237,21 @@ __global__ void __launch_bounds__(512) k_xpass_rhs(Dims d, typename Vec<T>::t* I
         VT* urow = Iu + (size_t)yy * d.ldI;
         VT* vrow = Iv + (size_t)yy * d.ldI;
         build_pair(Z, urow, vrow, d, lane, active);
-        fft_run<true>(Z, d, lane, tw);
+        fft_run<true, kElemsPerThread, true>(Z, d, lane, tw);
         for (int n = lane; n < d.M; n += d.Tg) {
             const VT z = Z[n];
             const T s = h ? W[n].y : W[n].x;
             Z[n] = mk<VT>(z.x * s, z.y * s);
         }
         fft_run<false>(Z, d, lane, tw);
-        extract_pair(Z, urow, vrow, d, lane, active, scale);
+        bool done = false;
+        if constexpr (sizeof(T) == 8) {
+            const FxMean zm = fx_mean(g);
+            done = zm.out || wm.out;
+            if (done && active)
+                extract_pair_rhs(Z, urow, vrow, Iw + (size_t)yy * d.ldI, d, lane, scale, zm.m, h ? wm.m.y : wm.m.x);
+        }
+        if (!done) extract_pair(Z, urow, vrow, d, lane, active, scale);
         __syncthreads();
     }
 }
@@ -265,7 +281,7 @@ __global__ void __launch_bounds__(512) k_xpass_rhs3(Dims d, typename Vec<T>::t* 
     VT* vrow = Iv + (size_t)(y1 + (role == 2)) * d.ldI;
     build_pair<E>(Z, role ? urow : Iw + (size_t)y1 * d.ldI, role ? vrow : Iw + (size_t)(y1 + 1) * d.ldI, d, lane,
                   active);
-    fft_run<true, E>(Z, d, lane, tw);
+    fft_run<true, E, true>(Z, d, lane, tw);
     if (role) {
         for (int n = lane; n < d.M; n += d.Tg) {
             const VT z = Z[n];
@@ -274,6 +290,15 @@ __global__ void __launch_bounds__(512) k_xpass_rhs3(Dims d, typename Vec<T>::t* 
         }
     }
     fft_run<false, E>(Z, d, lane, tw);
+    if constexpr (sizeof(T) == 8) {
+        const FxMean zm = fx_mean(g), wm = fx_mean(g - role);
+        if (zm.out || wm.out) {
+            if (active && role)
+                extract_pair_rhs(Z, urow, vrow, Iw + (size_t)(y1 + (role == 2)) * d.ldI, d, lane, scale, zm.m,
+                                 role == 2 ? wm.m.y : wm.m.x);
+            return;
+        }
+    }
     extract_pair(Z, urow, vrow, d, lane, active && role, scale);
 }
 

@@ -92,6 +92,7 @@ Carve carve(const Dims& d, int ntab) {
 Launch shape(int Tg, size_t bytes_per_group, int max_smem) {
     Launch L{};
     int G = (256 / Tg) > 1 ? 256 / Tg : 1;
+    G = G < kFxGroups / 2 ? G : kFxGroups / 2;   // (the forward y-pass runs up to 2 G transforms at a time)
     while (G > 1 && (G * Tg > 512 || G * bytes_per_group > (size_t)max_smem / 2)) --G;
     L.G = G;
     L.threads = G * Tg;

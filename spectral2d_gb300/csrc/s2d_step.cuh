@@ -176,7 +176,8 @@ __device__ __forceinline__ void build_pair(VT* buf, const VT* __restrict__ X, co
 
 // Split the forward FFT P of p = a + i b (a, b real rows) into the half
 // spectra A(k) = (P(k) + conj P(M-k))/2 and B(k) = (P(k) - conj P(M-k))/(2i),
-// k in [0, K], times scale.
+// k in [0, K], times scale.  (Entry k of A and B is written by the thread that
+// reads buf[k].)
 template <typename VT>
 __device__ __forceinline__ void extract_pair(const VT* buf, VT* A, VT* B, const Dims& d, int lane,
                                              bool active, decltype(buf[0].x) scale) {
@@ -195,6 +196,51 @@ __device__ __forceinline__ void extract_pair(const VT* buf, VT* A, VT* B, const 
         const VT q = buf[k == 0 ? 0 : d.M - k];
         A[k] = mk<VT>((p.x + q.x) * scale, (p.y - q.y) * scale);
         B[k] = mk<VT>((p.y + q.y) * scale, (q.x - p.x) * scale);
+    }
+}
+
+// The products' parts that are linear in the fluctuations, where a row's means
+// m = (u0, v0) were left out of its transform (fx_constant_out): entry U, V of
+// the rows' half spectra (entry 0: mean) becomes what the split of the
+// fluctuations' products lacks.  f = 2 M scale, the split's weight of a mean
+// times a half spectrum.  Basdevant: u0 v' + v0 u' and 2 (v0 v' - u0 u'), the
+// means' own products in entry 0.
+__device__ __forceinline__ void linear_part_bas(double2& U, double2& V, double2 m, double f, bool mean) {
+    if (mean) {   // half the means: entry 0 counts once, not twice as the pair k, -k
+        U = make_double2(0.5 * m.x, 0.0);
+        V = make_double2(0.5 * m.y, 0.0);
+    }
+    const double fu = __dmul_rn(f, m.x), fv = __dmul_rn(f, m.y);
+    const double2 u = U, v = V;
+    U = make_double2(fma(fu, v.x, __dmul_rn(fv, u.x)), fma(fu, v.y, __dmul_rn(fv, u.y)));
+    V = make_double2(2.0 * fma(fv, v.x, -__dmul_rn(fu, u.x)), 2.0 * fma(fv, v.y, -__dmul_rn(fu, u.y)));
+}
+// Conservative: u0 w' + w0 u' + u0 w0 and v0 w' + w0 v' + v0 w0; a
+// mean that was not left out is zero here and part of the fluctuations.
+__device__ __forceinline__ void linear_part_rhs(double2& U, double2& V, double2 W, double2 m, double w0, double f,
+                                                bool mean) {
+    if (mean) {
+        U = make_double2(U.x - m.x, 0.0);
+        V = make_double2(V.x - m.y, 0.0);
+        W.y = 0.0;
+    }
+    const double fu = __dmul_rn(f, m.x), fv = __dmul_rn(f, m.y), fw = __dmul_rn(f, w0);
+    U = make_double2(fma(fu, W.x, __dmul_rn(fw, U.x)), fma(fu, W.y, __dmul_rn(fw, U.y)));
+    V = make_double2(fma(fv, W.x, __dmul_rn(fw, V.x)), fma(fv, W.y, __dmul_rn(fw, V.y)));
+}
+
+// extract_pair in place over the half spectra A and B that the products were
+// made from: part(k, A(k), B(k)) turns an entry into its linear part.
+template <typename Part>
+__device__ __forceinline__ void extract_pair_add(const double2* buf, double2* A, double2* B, const Dims& d, int lane,
+                                                 double scale, Part part) {
+#pragma unroll 1
+    for (int k = lane; k <= d.K; k += d.Tg) {
+        const double2 p = buf[k], q = buf[k == 0 ? 0 : d.M - k];
+        double2 a = __ldcg(&A[k]), b = __ldcg(&B[k]);
+        part(k, a, b);
+        A[k] = make_double2(fma(p.x + q.x, scale, a.x), fma(p.y - q.y, scale, a.y));
+        B[k] = make_double2(fma(p.y + q.y, scale, b.x), fma(q.x - p.x, scale, b.y));
     }
 }
 
@@ -217,12 +263,22 @@ __device__ __forceinline__ void xpass_bas_body(const Dims& d, typename Vec<T>::t
     VT* urow = Iu + (size_t)(active ? y : 0) * d.ldI;
     VT* vrow = Iv + (size_t)(active ? y : 0) * d.ldI;
     build_pair(Z, urow, vrow, d, lane, active);
-    fft_run<true>(Z, d, lane, tw);
+    fft_run<true, kElemsPerThread, true>(Z, d, lane, tw);
     for (int n = lane; n < d.M; n += d.Tg) {
         const VT z = Z[n];
         Z[n] = mk<VT>(z.x * z.y, z.y * z.y - z.x * z.x);
     }
     fft_run<false>(Z, d, lane, tw);
+    if constexpr (sizeof(T) == 8) {
+        const FxMean zm = fx_mean(g);
+        if (zm.out) {
+            if (active)
+                extract_pair_add(Z, urow, vrow, d, lane, scale, [&](int k, double2& U, double2& V) {
+                    linear_part_bas(U, V, zm.m, 2.0 * d.M * scale, k == 0);
+                });
+            return;
+        }
+    }
     extract_pair(Z, urow, vrow, d, lane, active, scale);
 }
 

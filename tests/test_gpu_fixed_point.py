@@ -152,3 +152,78 @@ def test_conservative_rhs_at_the_sizes_where_its_kernel_changes(mods, n, precisi
         dW = s.compute_rhs()
     ref, _ = O.compute_rhs(w, O.truncate(O.compute_psi(w, g), g), g, 0.01, round_trip=False)
     assert O.rel_l2(dW, O.truncate(ref, g)) < tol
+
+
+def _flow_of_y_and_perturbation(n, amp):
+    """A vorticity that depends on y alone, and a perturbation (kx > 0) of largest mode amp times its own."""
+    g = O.get_grid_size(n, n)
+    ky = np.fft.fftfreq(g.nyG, 1.0 / g.nyG)
+    base = np.zeros((g.nyG, g.cISize), complex)
+    base[np.abs(ky) == 4, 0] = 2.0
+    pert = O.truncate(O.random_state(g, 3, decay=0.2), g)
+    pert[:, 0] = 0
+    return g, base, pert * (2.0 * amp / np.abs(pert).max())
+
+
+def _perturbed_tendency(g, base, pert, form):
+    """The inviscid tendency of base + pert from the products of base and perturbation, formed apart (so that its errors
+    are relative to the perturbation), and the bounds on the 2-norm of a right-hand side's error in kx > 0 and in kx = 0:
+    _transform_bound with the products that are linear in the perturbation, and with the quadratic ones."""
+    M, K = g.nxG, g.nx // 2
+    kx = np.arange(g.cISize)[None, :]
+    ky = np.fft.fftfreq(M, 1.0 / M)[:, None]
+    phys = lambda f: np.fft.irfft(np.fft.ifft(f, axis=0) * M, n=M, axis=1) * M   # noqa: E731
+    spec = lambda p: np.fft.rfft2(p) / M ** 2                                   # noqa: E731
+    norm = lambda *ps: sum(np.linalg.norm(spec(p)) for p in ps)                 # noqa: E731
+    psi0, psi1 = (O.truncate(O.compute_psi(w, g), g) for w in (base, pert))
+    u0, w0 = phys(1j * ky * psi0), phys(base)
+    u1, v1, w1 = phys(1j * ky * psi1), phys(-1j * kx * psi1), phys(pert)
+    lin = -1j * kx * spec(u0 * w1 + w0 * u1) - 1j * ky * spec(v1 * w0)
+    lin[:, 0] = 0   # its x-means vanish
+    dW = O.truncate(lin - 1j * kx * spec(u1 * w1) - 1j * ky * spec(v1 * w1), g)
+    if form == "basdevant":
+        weight, linear, quad = K * K, norm(u0 * v1, 2 * u0 * u1), norm(u1 * v1, v1 * v1 - u1 * u1)
+    else:
+        weight, linear, quad = K, norm(u0 * w1, w0 * u1, v1 * w0), norm(u1 * w1, v1 * w1)
+    per = 2 * 6 * 2e-16 * weight
+    return dW, per * (linear + quad), per * quad
+
+
+# plan 2 (FP64): the general transform; 64 | 768: 4 and 12 elements per thread,
+# three groups and one; amp 0.1: the means stay in the transforms, or not, row by row
+@pytest.mark.parametrize("form", ["basdevant", "conservative"])
+@pytest.mark.parametrize("plan", [0, 2])
+@pytest.mark.parametrize("amp", [0.1, 1e-3, 1e-6, 1e-10])
+@pytest.mark.parametrize("n", [64, 96, 768])
+def test_weak_perturbations_keep_their_bits_beside_a_large_mean(mods, n, amp, plan, form):
+    """An FP64 transform of u + i v adds a row's mean u in butterflies without
+    twiddles, so a weak v keeps its own 53 bits; ky = 0 and kx = 0 (in which
+    the base flow has no linear term of u u) show it."""
+    _, S2D = mods
+    g, base, pert = _flow_of_y_and_perturbation(n, amp)
+    ref, bound, bound0 = _perturbed_tendency(g, base, pert, form)
+    with S2D(n, nu=0.0, nonlinear_form=form) as s:
+        s.fft_plan = plan
+        s.set_state(base)
+        alone = s.compute_rhs()
+        s.set_state(base + pert)
+        dW = s.compute_rhs()
+    assert np.all(alone == 0.0)
+    err = dW - ref
+    assert np.linalg.norm(err[:, 1:]) <= bound
+    if amp <= 1e-3:   # (else not all rows' means stand apart)
+        assert np.linalg.norm(err[:, 0]) <= bound0
+        assert np.all(np.abs(err[0, 1:5]) <= 5e-14 * np.abs(ref[0, 1:5]))
+
+
+def test_a_batch_and_a_run_alone_agree_beside_a_large_mean(mods):
+    Ensemble, S2D = mods
+    for n, amp in ((64, 1e-6), (128, 0.1)):
+        _, base, pert = _flow_of_y_and_perturbation(n, amp)
+        with Ensemble([n], [1e-3]) as ens, S2D(n, nu=1e-3) as s:
+            ens.runs[0].set_state(base + pert)
+            ens.set_dt([1e-3])
+            ens.integrate_steps(2)
+            s.set_state(base + pert)
+            s.integrate_steps(2, 1e-3)
+            assert np.array_equal(ens.runs[0].get_state()[0], s.get_state()[0])
