@@ -429,6 +429,8 @@ __device__ __forceinline__ fx2 fx_from(double2 z, int emax, int n0) {
                fx_from(__double2hiint(z.y), (unsigned)__double2loint(z.y), emax, n0)};
 }
 __device__ __forceinline__ double2 fx_to(fx2 z, int eb) {
+    if (eb < 64 || eb > 2046)   // uniform over a transform
+        return make_double2(__longlong_as_double(fx_to_wide(z.x, eb)), __longlong_as_double(fx_to_wide(z.y, eb)));
     return make_double2(__longlong_as_double(fx_to(z.x, eb)), __longlong_as_double(fx_to(z.y, eb)));
 }
 __device__ __forceinline__ fx2 fx_ld(const longlong2* buf, int i) {

@@ -228,10 +228,10 @@ S2D_HD int fx_exponent_base(int emax, int n0, int t) { return emax >= 0x7FF ? 1 
 
 // x -> FP64 bits, x 2^(eb - 1086) rounded to nearest; eb from
 // fx_exponent_base.  A result above FP64's range is an infinity, one below its
-// normal range zero.  The conversion instruction runs at 2 per cycle and SM
-// like all FP64, but beside the integer work, and the exponent is added to its
-// result's high word: 5 instructions, where normalising and rounding with
-// integer operations took 32.
+// normal range zero: the kernels take fx_to_wide for such eb.  The conversion
+// instruction runs at 2 per cycle and SM like all FP64, but beside the integer
+// work, and the exponent is added to its result's high word: 5 instructions,
+// where normalising and rounding with integer operations took 32.
 S2D_HD long long fx_to(long long x, int eb) {
     const double v = (double)x;
 #ifdef __CUDA_ARCH__
@@ -250,6 +250,34 @@ S2D_HD long long fx_to(long long x, int eb) {
         if (eb >= 1 << 16) g = 0x7FF80000, k = 0;
     }
     return (long long)(((unsigned long long)(unsigned)g << 32) | k);
+}
+
+// The same where the exponent may leave [1, 2046] (eb < 64 or eb > 2046):
+// gradual below the normal range, as FP64 arithmetic is.  (double)x is exact or
+// rounded once; of the two powers of two only the second can round.  (As a
+// product with one factor after fx_to the compiler makes it every result's:
+// 2048^2 1787 -> 1833 us per step.)
+S2D_HD double fx_pow2(int e) {   // -1022 <= e <= 1023
+    const long long b = (long long)(e + 1023) << 52;
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double(b);
+#else
+    double v;
+    __builtin_memcpy(&v, &b, 8);
+    return v;
+#endif
+}
+S2D_HD long long fx_to_wide(long long x, int eb) {
+    const int s = eb - 1086;
+    const int a = s < -960 ? -960 : (s > 960 ? 960 : s), r = s - a;
+    const double v = (double)x * fx_pow2(a) * fx_pow2(r < -1022 ? -1022 : (r > 1023 ? 1023 : r));
+#ifdef __CUDA_ARCH__
+    const long long b = __double_as_longlong(v);
+#else
+    long long b;
+    __builtin_memcpy(&b, &v, 8);
+#endif
+    return eb >= 1 << 16 ? 0x7FF8000000000000LL : b;
 }
 
 // Magnitude bound of an element for the sum: |x| + |y| >= |z| of the high

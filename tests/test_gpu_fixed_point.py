@@ -227,3 +227,28 @@ def test_a_batch_and_a_run_alone_agree_beside_a_large_mean(mods):
             s.set_state(base + pert)
             s.integrate_steps(2, 1e-3)
             assert np.array_equal(ens.runs[0].get_state()[0], s.get_state()[0])
+
+
+@pytest.mark.parametrize("form", ["basdevant", "conservative"])
+@pytest.mark.parametrize("plan", [0, 2])
+@pytest.mark.parametrize("n", [64, 576, 768])
+def test_results_below_the_normal_range_are_gradual(mods, n, plan, form):
+    """w 2^k, k chosen so that the products' spectra are subnormal numbers: 2^(2k) times the right-hand side to the
+    rounding of the x-pass's results and of K3's, half of 2^-1074 each: M rows are summed, and a mode's two products
+    weighed by up to K^2 (four parts, real and imaginary)."""
+    _, S2D = mods
+    g = O.get_grid_size(n, n)
+    w = O.truncate(O.random_state(g, 5, decay=0.1), g)
+    with S2D(n, nu=0.0, nonlinear_form=form) as s:
+        s.fft_plan = plan
+        s.set_state(w)
+        dW = s.compute_rhs()
+        k = -int((1040 + np.log2(np.abs(dW).max())) / 2)
+        s.set_state(w * 2.0 ** k)
+        low = s.compute_rhs()
+    K = n // 2
+    weight = K * K if form == "basdevant" else K
+    ulp = 2.0 ** -1074
+    want = dW * 2.0 ** k * 2.0 ** k
+    assert np.abs(want).max() > 1000 * weight * ulp
+    assert np.abs(low - want).max() <= 4 * weight * (g.nxG / 2 + 1) * ulp
