@@ -506,3 +506,67 @@ def test_fused_forward_at_the_edges_of_its_tiles(S, grid, B):
         yl = net.forward(x)
     assert _rel(yf, yl) < 2e-3
     assert np.abs(yf - yl).max() / np.sqrt(np.mean(yl.astype(np.float64) ** 2)) < 2e-2
+
+
+@pytest.mark.parametrize("grid, B", [(30, 80), (31, 80), (61, 24), (192, 3)])
+def test_both_tile_forms_of_the_fused_forward_give_the_same_bits(S, grid, B):
+    """B images together are more than six small tiles per SM (pixel pairs), each alone fewer (pixels)."""
+    x = np.random.default_rng(5).standard_normal((B, grid, grid, 2)).astype(np.float32)
+    with S.ClosureNet(grid, max_batch=B, seed=3) as net:
+        net.set_scales([1.0, 1.0, 1.0])
+        y = net.forward(x)
+        for b in (0, 1, B - 1):
+            assert np.array_equal(net.forward(x[b:b + 1])[0], y[b])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_les_batch_on_pixel_pairs_equals_the_runs_alone(S, precision):
+    """Three runs of 128^2 take the pair form of the fused forward, one the pixel form."""
+    n, nu, steps, dt = 128, 1e-3, 3, 2e-3
+    w0 = [O.random_state(O.get_grid_size(n, n), 50 + i, decay=0.2) for i in range(3)]
+    with S.ClosureNet(192, max_batch=3, seed=13) as net:
+        net.set_scales([1.0, 1.0, 0.05])
+        with S.Ensemble([n] * 3, [nu] * 3, precision=precision) as ens:
+            for r, w in zip(ens.runs, w0):
+                r.set_state(w)
+            ens.set_dt([dt] * 3)
+            ens.set_closure(net)
+            ens.integrate_steps(steps)
+            ens.status()
+            wb = [r.get_state()[0] for r in ens.runs]
+            ens.set_closure(None)
+        for i in (0, 2):
+            with S.Spectral2D(n, nu=nu, precision=precision) as a:
+                a.set_state(w0[i])
+                S.les_set_closure(a, net)
+                S.les_integrate_steps(a, steps, dt)
+                assert np.array_equal(a.get_state()[0], wb[i])
+                S.les_set_closure(a, None)
+
+
+def test_paired_and_scalar_activations_give_the_same_bits(S):
+    """A channel beyond the paired form's bound sends its group of eight to the
+    scalar form: the other channels' activations and gradients stay the same.
+    (The layers after see the odd channel with zero weights.)"""
+    grid, B = 24, 2
+    rng = np.random.default_rng(11)
+    with S.ClosureNet(grid, max_batch=B, seed=3) as net:
+        net.set_scales([1.0, 1.0, 1.0])
+        net.keep_layer_grads(True)
+        p = net.get_params().copy()
+        odd = 8 * np.arange(4) + 7
+        W1 = p[608:608 + 32 * 9 * 32].reshape(32, 9, 32)
+        W1[:, :, odd] = 0
+        x = (4.0 * rng.standard_normal((B, grid, grid, 2))).astype(np.float32)
+        t = rng.standard_normal((B, grid, grid)).astype(np.float32)
+        out = []
+        for bias in (0.0, 1000.0):
+            p[32 * 9 * 2 + odd] = bias
+            net.set_params(p)
+            net.grad(x, t)
+            out.append([net.tensor(k, l, B) for k, l in ((1, 0), (0, 1), (2, 0))])
+    rest = np.setdiff1d(np.arange(32), odd)
+    groups = [np.abs(o[0]).reshape(B, grid, grid, 4, 8).max(-1) for o in out]
+    assert np.mean(groups[0] < 12.5) > 0.5 and groups[1].min() > 12.5   # paired mostly; scalar throughout
+    for a, b in zip(*out):
+        assert np.array_equal(a[..., rest], b[..., rest])

@@ -86,3 +86,30 @@ def test_state_arrays_at_half_an_element(S, n, mem):
     assert np.array_equal(d, dW)
     for a, b in ((gw, w1), (gp, p1), (hw, w1), (hp, p1)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("mem", ["pageable", "pinned", "fresh"])
+def test_closure_batches_through_staging_copies(S, mem, monkeypatch):
+    """S2D_HOST_IO=copy: a batch smaller than the network's through the staging
+    buffer and the copy-out, bit for bit what arrays in place give; and (without
+    it) an input whose pages are not resident, staged beside one in place."""
+    from spectral2d_gb300 import _lib as L
+    from spectral2d_gb300.solver import _fptr
+    rng = np.random.default_rng(3)
+    x = rng.standard_normal((3, 24, 24, 2)).astype(np.float32)
+    t = rng.standard_normal((3, 24, 24)).astype(np.float32)
+    if mem == "fresh":
+        x = np.zeros_like(x)
+    out = []
+    for io in ("in_place", "copy"):
+        if io == "copy":
+            monkeypatch.setenv("S2D_HOST_IO", "copy")
+        with S.ClosureNet(24, max_batch=5, seed=1) as net:
+            net.set_scales([2.0, 0.5, 0.25])
+            xs = np.zeros(x.shape, np.float32) if mem == "fresh" else _at(x, 0, mem)
+            loss, g = net.grad(xs, _at(t, 0, "pageable" if mem == "fresh" else mem))
+            y = _at(np.full_like(t, np.nan), 0, "pinned" if mem == "pinned" else "pageable")
+            L.check(net._L.s2d_cnn_forward_host(net._c, _fptr(xs), 3, _fptr(y)))
+            out.append((loss, g, y.copy()))
+    assert out[0][0] == out[1][0]
+    assert np.array_equal(out[0][1], out[1][1]) and np.array_equal(out[0][2], out[1][2])
