@@ -252,3 +252,22 @@ def test_results_below_the_normal_range_are_gradual(mods, n, plan, form):
     want = dW * 2.0 ** k * 2.0 ** k
     assert np.abs(want).max() > 1000 * weight * ulp
     assert np.abs(low - want).max() <= 4 * weight * (g.nxG / 2 + 1) * ulp
+
+
+@pytest.mark.parametrize("n", [8, 64, 96])
+def test_the_allocation_free_rhs_keeps_weak_perturbations_too(built_lib, n):
+    """Its x-pass scales the products itself (u and v come unscaled); 8^2: one
+    thread per transform, 32 of them in a CTA."""
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+
+    from spectral2d_gb300 import _lib as L
+    g, base, pert = _flow_of_y_and_perturbation(n, 1e-6)
+    ref, bound, bound0 = _perturbed_tendency(g, base, pert, "basdevant")
+    w = torch.from_numpy((base + pert).view(np.float64).copy()).cuda()
+    dW = torch.full_like(w, float("nan"))
+    torch.cuda.synchronize()
+    assert L.lib().s2d_compute_rhs_noalloc(n, 0.0, C.c_void_p(w.data_ptr()), C.c_void_p(dW.data_ptr()), None) == 0
+    torch.cuda.synchronize()
+    err = dW.cpu().numpy().view(np.complex128).reshape(ref.shape) - ref
+    assert np.linalg.norm(err[:, 1:]) <= bound and np.linalg.norm(err[:, 0]) <= bound0
