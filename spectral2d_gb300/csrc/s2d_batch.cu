@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 && !X32 ? 2 : 1) k_batch_s
                     fx_yinv_body<12>(R.d, S, R.rk2, fs, (const FxTw*)R.tw, R.G12, blk, bufs);
                 else f32_yinv_body<12>(R.d, S, R.rk2, fs, R.tw, R.G12, blk, bufs);
             } else if (ph == 1) {
-                bool done = false;
+                bool row32 = false;
                 if constexpr (sizeof(T) == 4 && X32) {
                     // FP32 rows of M = 3072: the register radix-12/16 x-pass of
                     // the single run (k_xpass32), one row per 256 threads
@@ -132,16 +132,14 @@ __global__ void __launch_bounds__(512, sizeof(T) == 4 && !X32 ? 2 : 1) k_batch_s
                         const int g = threadIdx.x / 256, y = blk * R.G12 + g;
                         xpass32_m3072_row(R.d, R.I0, R.I1, R.tw, y, y < R.d.rows && g < R.G12,
                                           threadIdx.x - g * 256, bufs + (size_t)g * kX32Buf);
-                        done = true;
+                        row32 = true;
                     }
                 }
-                if (done) {
-                } else if (!R.d.direct) {
-                    xpass_bas_body<T>(R.d, R.I0, R.I1, R.tw, R.G12, (T)1, blk, bufs);
-                } else if constexpr (sizeof(T) == 8) {
-                    fx_xpass_body<12>(R.d, R.I0, R.I1, (const FxTw*)R.tw, R.G12, 1.0, blk, bufs);
-                } else {
-                    f32_xpass_body<12>(R.d, R.I0, R.I1, R.tw, R.G12, 1.f, blk, bufs);
+                if (!row32) {
+                    if (!R.d.direct) xpass_bas_body<T>(R.d, R.I0, R.I1, R.tw, R.G12, (T)1, blk, bufs);
+                    else if constexpr (sizeof(T) == 8)
+                        fx_xpass_body<12>(R.d, R.I0, R.I1, (const FxTw*)R.tw, R.G12, 1.0, blk, bufs);
+                    else f32_xpass_body<12>(R.d, R.I0, R.I1, R.tw, R.G12, 1.f, blk, bufs);
                 }
             } else {
                 if (!R.d.direct)

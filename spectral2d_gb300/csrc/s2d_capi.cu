@@ -335,7 +335,7 @@ struct CopyStreamJoin {
 
 // Reference-layout outputs: the retained rectangle written in place by the
 // conversion kernel, or into the staging arrays and copied; the rest by
-// send_zeros, which the caller issues first.
+// send_zeros, whose kernel and copies the caller issues before this.
 int download_ref(s2d_handle* h, const void* S, const HostArray& w, const HostArray& p) {
     if (!w.host && !p.host) return S2D_OK;
     if ((w.host && !w.dev) || (p.host && !p.dev)) S2D_TRY(ensure_ref_stage(h));
@@ -635,7 +635,7 @@ int s2d::create_handle(const s2d_config* cfg, cudaStream_t ext_stream, s2d_handl
         return bail(fail(S2D_ERR_CUDA, "rk2 init failed"));
 
     // launch shapes: about 256 threads per CTA so that at least two CTAs
-    // share an SM and one CTA's barrier phases overlap the other's FP64 work
+    // share an SM and one CTA's barrier phases overlap the other's arithmetic
     const size_t tb = (size_t)d.M * h->vsz;
     const int tgt = 256;
     int rr;

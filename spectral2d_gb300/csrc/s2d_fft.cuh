@@ -1,14 +1,15 @@
 // s2d_fft.cuh -- block-level mixed-radix Stockham FFT in shared memory.
 //
-// One transform of length M is owned by Tg = M/12 consecutive threads; a CTA
-// runs several transforms of the same length side by side.  Each pass with
+// One transform of length M is owned by Tg = M/E consecutive threads, E = 12 or
+// (small grids) 4 elements each; a CTA runs several transforms of the same
+// length side by side.  Each pass with
 // radix R is the self-sorting Stockham step (Govindaraju et al., SC'08):
 // butterfly j (0 <= j < M/R) reads x[j + r*M/R], multiplies by the twiddle
 // w^(r*(j mod Ns)*M/(Ns*R)) with w = exp(-2 pi i/M), does a radix-R DFT and
 // writes x[(j/Ns)*Ns*R + j mod Ns + r*Ns], Ns being the product of the
-// earlier radices.  The pass is done in place: every thread first loads all
-// 12 of its elements into registers, the CTA synchronises, then every thread
-// writes its results.
+// earlier radices.  The pass is done in place: every thread first loads all of
+// its elements into registers, the CTA synchronises, then every thread writes
+// its results.
 //
 // FP64 values are transformed in 64-bit block fixed point on the integer
 // pipes (fx_run below; the arithmetic is in s2d_fixed.cuh): the first pass
@@ -124,8 +125,8 @@ __device__ __forceinline__ void butterfly(VT* v) {
 // j mod Ns by a multiply-high: q = floor(j mg / 2^32) with mg = ceil(2^32 /
 // Ns) (Dims::mg, set on the host) is floor(j / Ns) exactly while
 // j (mg Ns - 2^32) < 2^32, i.e. for every j < 2^32 / Ns (here j < M <= 6144).
-// No integer division on the device: on GB300 it competes with the FP64
-// pipe (the FP64 step ran 3 % faster without one per butterfly).
+// No integer division on the device: about 20 instructions per butterfly, on
+// the integer pipes that the FP64 transforms are bound by.
 struct ModNs {
     int Ns;
     unsigned mg;

@@ -243,7 +243,6 @@ struct Kern {
     // fu = ky * rk2, fv = -kx * rk2 per mode: the factors OP_U / OP_V form
     // in the kernel, as tables (the same products, so the same bits)
     static cudaError_t init_uv_factors(const Dims& d, const double* rk2, double* fu, double* fv, cudaStream_t st);
-    static size_t smem_limit_yinv();
 };
 
 }  // namespace s2d

@@ -122,9 +122,10 @@ __global__ void __launch_bounds__(256) k_stage(Dims d, const typename Vec<T>::t*
 // ---- FP64, direct plans (s2d_fxstep.cuh) ---------------------------------
 // E elements per thread: 12, or 4 for small grids.  CTAs of at most 256
 // threads: three per SM (B = 1, 80 registers); up to 384: two (B = 3, 80; one
-// at 128: the 3072^2 step 5.77 -> 5.50 ms, 4.84 with the results' conversion); up to 512: K1 two
-// (B = 2, 64), whose loads and stores gain more than its spills cost (4096^2
-// 2.37 -> 2.31 ms), K2 and K3 one (B = 0, 128; two: 4.5 -> 5.0, 2.8 -> 3.3 ms).
+// at 128: the 3072^2 step 5.77 -> 5.50 ms, 4.57 now); up to 512: K1 two (B = 2,
+// 64), whose loads and stores gain more than its spills cost (4096^2 2.37 ->
+// 2.31 ms, 1.89 with the twiddles read ahead), K2 and K3 one (B = 0, 128; two:
+// 4.5 -> 5.0, 2.8 -> 3.3 ms).
 template <int E, int B>
 __global__ void __launch_bounds__(kMaxThreads<B>, (kMinBlocks<double, B>))
     k_fx_yinv(Dims d, const double2* __restrict__ S, const double* __restrict__ rk2, FieldSet fs,
@@ -1008,11 +1009,6 @@ template <typename T>
 cudaError_t Kern<T>::init_stage_factors(const Dims& d, double nu, double* cc, double* vk, cudaStream_t st) {
     k_init_stage_factors<<<grid_for((long)d.KX * d.KY, 256), 256, 0, st>>>(d, nu, (double2*)cc, vk);
     return cudaGetLastError();
-}
-
-template <typename T>
-size_t Kern<T>::smem_limit_yinv() {
-    return 0;
 }
 
 template struct Kern<double>;

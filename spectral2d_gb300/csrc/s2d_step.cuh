@@ -135,7 +135,7 @@ __device__ __forceinline__ void yinv_body(const Dims& d, const typename Vec<T>::
 
     VT* out = reinterpret_cast<VT*>(outp);
     const int gtot = min(G, d.KX - kx0);
-    if (G == 1) {   // no integer division per element (it competes with the FP64 pipe)
+    if (G == 1) {   // no index split per element
         for (int y = threadIdx.x; y < d.M; y += blockDim.x) out[(size_t)y * d.ldI + kx0] = bufs[y];
     } else {
         const DivBy byG(G);
