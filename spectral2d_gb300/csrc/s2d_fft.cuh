@@ -429,10 +429,12 @@ __device__ __forceinline__ fx2 fx_from(double2 z, int emax, int n0) {
     return fx2{fx_from(__double2hiint(z.x), (unsigned)__double2loint(z.x), emax, n0),
                fx_from(__double2hiint(z.y), (unsigned)__double2loint(z.y), emax, n0)};
 }
-__device__ __forceinline__ double2 fx_to(fx2 z, int eb) {
-    if (eb < 64 || eb > 2046)   // uniform over a transform
-        return make_double2(__longlong_as_double(fx_to_wide(z.x, eb)), __longlong_as_double(fx_to_wide(z.y, eb)));
-    return make_double2(__longlong_as_double(fx_to(z.x, eb)), __longlong_as_double(fx_to(z.y, eb)));
+// n: fx_normal_base of the results' exponent base eb.  Where they differ, which
+// is rare, the kernels multiply their results by fx_rest(eb) afterwards or in a
+// copy of the last pass (beside each conversion every row pays for it: 2048^2
+// 1770 us per step, 1787 with a branch there, 1833 with the product).
+__device__ __forceinline__ double2 fx_to(fx2 z, int n) {
+    return make_double2(__longlong_as_double(fx_to_normal(z.x, n)), __longlong_as_double(fx_to_normal(z.y, n)));
 }
 __device__ __forceinline__ fx2 fx_ld(const longlong2* buf, int i) {
     const longlong2 z = buf[i];
@@ -514,6 +516,7 @@ __device__ __forceinline__ void fx_pass(longlong2* buf, int M, int Ns, unsigned 
     }
     __syncthreads();
     const ModNs mod(Ns, mg);
+    const int n = LAST ? fx_normal_base(eb) : 0;
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
         const int j = lane + b * T;
@@ -525,13 +528,23 @@ __device__ __forceinline__ void fx_pass(longlong2* buf, int M, int Ns, unsigned 
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             if constexpr (LAST) {
-                double2 z = fx_to(v[b][r], eb);
-                if (INV && c) z = make_double2(z.x + c->x, z.y + c->y);
+                const double2 z = fx_to(v[b][r], n);
                 buf[base + r * Ns] = make_longlong2(__double_as_longlong(z.x), __double_as_longlong(z.y));
             } else {
                 fx_st(buf, base + r * Ns, v[b][r]);
             }
         }
+    }
+    if (LAST && (n != eb || c)) {   // this thread's results again (Ns = M / R: element j + r Ns)
+        const double f = fx_rest(eb);
+        const double2 a = c ? *c : make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int i = lane; i < stride; i += T)
+#pragma unroll 1
+            for (int e = i; e < M; e += stride) {
+                double2* z = reinterpret_cast<double2*>(buf) + e;
+                *z = make_double2(fma(z->x, f, a.x), fma(z->y, f, a.y));
+            }
     }
     __syncthreads();
 }

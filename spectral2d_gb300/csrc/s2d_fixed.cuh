@@ -226,13 +226,12 @@ S2D_HD long long fx_from(int hi, unsigned lo, int emax, int n0) {
 // infinity or NaN.
 S2D_HD int fx_exponent_base(int emax, int n0, int t) { return emax >= 0x7FF ? 1 << 16 : emax + n0 + 1 + t; }
 
-// x -> FP64 bits, x 2^(eb - 1086) rounded to nearest; eb from
-// fx_exponent_base.  A result above FP64's range is an infinity, one below its
-// normal range zero: the kernels take fx_to_wide for such eb.  The conversion
-// instruction runs at 2 per cycle and SM like all FP64, but beside the integer
-// work, and the exponent is added to its result's high word: 5 instructions,
-// where normalising and rounding with integer operations took 32.
-S2D_HD long long fx_to(long long x, int eb) {
+// x -> FP64 bits, x 2^(eb - 1086) rounded to nearest, for 64 <= eb <= 2046: zero
+// or in the normal range.  The conversion instruction runs at 2 per cycle and SM
+// like all FP64, but beside the integer work, and the exponent is added to its
+// result's high word: 5 instructions, where normalising and rounding with
+// integer operations took 32.
+S2D_HD long long fx_to_normal(long long x, int eb) {
     const double v = (double)x;
 #ifdef __CUDA_ARCH__
     const int h = __double2hiint(v), l = __double2loint(v);
@@ -241,24 +240,17 @@ S2D_HD long long fx_to(long long x, int eb) {
     __builtin_memcpy(&vb, &v, 8);
     const int h = (int)(vb >> 32), l = (int)vb;
 #endif
-    int g = h ? h + (int)((unsigned)(eb - 1086) << 20) : 0;
-    unsigned k = (unsigned)l;
-    if (eb < 64 || eb > 2046) {   // uniform over a transform: the exponent may leave [1, 2046]
-        const int E = ((h >> 20) & 0x7FF) + eb - 1086;
-        if (E < 1) g = 0, k = 0;
-        if (E > 2046 && h) g = (h & 0x80000000) | 0x7FF00000, k = 0;
-        if (eb >= 1 << 16) g = 0x7FF80000, k = 0;
-    }
-    return (long long)(((unsigned long long)(unsigned)g << 32) | k);
+    const int g = h ? h + (int)((unsigned)(eb - 1086) << 20) : 0;
+    return (long long)(((unsigned long long)(unsigned)g << 32) | (unsigned)l);
 }
-
-// The same where the exponent may leave [1, 2046] (eb < 64 or eb > 2046):
-// gradual below the normal range, as FP64 arithmetic is.  (double)x is exact or
-// rounded once; of the two powers of two only the second can round.  (As a
-// product with one factor after fx_to the compiler makes it every result's:
-// 2048^2 1787 -> 1833 us per step.)
-S2D_HD double fx_pow2(int e) {   // -1022 <= e <= 1023
-    const long long b = (long long)(e + 1023) << 52;
+// An eb of fx_exponent_base brought into that range, and the power of two that
+// the results then lack: a product that overflows to infinity or underflows
+// gradually with one rounding, as FP64 arithmetic does; NaN for an input with an
+// infinity or NaN.  (With less than 2^-1022 every result is zero.)
+S2D_HD int fx_normal_base(int eb) { return eb < 64 ? 64 : (eb > 2046 ? 2046 : eb); }
+S2D_HD double fx_rest(int eb) {
+    const int d = eb - fx_normal_base(eb), r = d < -1022 ? -1022 : (d > 1023 ? 1023 : d);
+    const long long b = eb >= 1 << 16 ? 0x7FF8000000000000LL : (long long)(r + 1023) << 52;
 #ifdef __CUDA_ARCH__
     return __longlong_as_double(b);
 #else
@@ -267,17 +259,17 @@ S2D_HD double fx_pow2(int e) {   // -1022 <= e <= 1023
     return v;
 #endif
 }
-S2D_HD long long fx_to_wide(long long x, int eb) {
-    const int s = eb - 1086;
-    const int a = s < -960 ? -960 : (s > 960 ? 960 : s), r = s - a;
-    const double v = (double)x * fx_pow2(a) * fx_pow2(r < -1022 ? -1022 : (r > 1023 ? 1023 : r));
-#ifdef __CUDA_ARCH__
-    const long long b = __double_as_longlong(v);
-#else
-    long long b;
-    __builtin_memcpy(&b, &v, 8);
-#endif
-    return eb >= 1 << 16 ? 0x7FF8000000000000LL : b;
+
+// One result by itself, flushed to zero below the normal range.
+S2D_HD long long fx_to(long long x, int eb) {
+    const int n = fx_normal_base(eb);
+    const long long t = fx_to_normal(x, n);
+    if (n == eb) return t;
+    const int e = (int)((unsigned long long)t >> 52 & 0x7FF) + eb - n;
+    if (eb >= 1 << 16) return 0x7FF8000000000000LL;
+    if (e < 1 || x == 0) return 0;
+    const long long sign = t & (long long)0x8000000000000000ULL;
+    return e > 2046 ? sign | 0x7FF0000000000000LL : (t & (long long)0x800FFFFFFFFFFFFFULL) | (long long)e << 52;
 }
 
 // Magnitude bound of an element for the sum: |x| + |y| >= |z| of the high

@@ -101,9 +101,14 @@ __device__ __forceinline__ void fx_yinv_body(const Dims& d, const double2* __res
 
     // last pass, radix 4 (Ns = M / 4): results y = j + r M / 4 to the rows
     const int tn = max(t, fx_shift_total(M, per, sum, kFxByLimit));
-    const int eb = fx_exponent_base(emax, 3, tn);
+    const int eb = fx_exponent_base(emax, 3, tn), n = fx_normal_base(eb);
     const FxTw* tp = tw + d.twoff[d.npass - 1];
     double2* out = reinterpret_cast<double2*>(outp) + kx;
+    // (results that need more work: to the buffer, whose elements this thread has
+    // read; one store either way, so that others pay for no branch)
+    const bool park = n != eb;
+    double2* to = park ? reinterpret_cast<double2*>(buf) : out;
+    const int ld = park ? 1 : d.ldI;
 #pragma unroll
     for (int b = 0; b < kFxNB<E, 4>; ++b) {
         const int j = lane + b * T;
@@ -114,8 +119,13 @@ __device__ __forceinline__ void fx_yinv_body(const Dims& d, const double2* __res
         fx_bf4<true>(v);
         if (active) {
 #pragma unroll
-            for (int r = 0; r < 4; ++r) out[(size_t)(j + r * (M / 4)) * d.ldI] = fx_to(v[r], eb);
+            for (int r = 0; r < 4; ++r) to[(size_t)(j + r * (M / 4)) * ld] = fx_to(v[r], n);
         }
+    }
+    if (active && park) {   // (T divides M / 4: the rows lane + i T are this thread's)
+        const double f = fx_rest(eb);
+#pragma unroll 1
+        for (int y = lane; y < M; y += T) out[(size_t)y * d.ldI] = make_double2(to[y].x * f, to[y].y * f);
     }
 }
 
@@ -132,8 +142,11 @@ __device__ __forceinline__ void fx_yinv_body(const Dims& d, const double2* __res
 // Where the row's means (kx = 0) would take bits from the rest
 // (fx_constant_out) they are left out of the transforms, and the products'
 // parts that are linear in the rest are added in FP64 (linear_part_bas): at
-// the end, in a copy of the last pass, so that other rows' carries no more
-// than a branch (in one copy: 2048^2 K2 833 -> 880 us per step).
+// the end, in a copy of the last pass, so that other rows pay for no more than
+// one branch (2048^2 K2: 824 us per step; in one copy 880, with the results
+// parked in the buffer 836, by one store through a chosen pointer 830 and 4689
+// against 4501 at 4096^2).  The copy also takes results whose exponents leave
+// the normal range (fx_rest).
 // scale: factor of the results (1 when u and v are prescaled).
 template <int E>
 __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double2* Iv, const FxTw* __restrict__ tw,
@@ -285,18 +298,24 @@ __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double
     // ---- forward, last pass (radix 3, Ns = K): P(j), P(j + 2K); the split
     const int tf = max(t, fx_shift_total(M, per, sum, 2.0f * kFxByLimit));
     if (ebp < 1 << 16) ebp += tf;
+    const int n = fx_normal_base(ebp);
     const FxTw* tp = tw + d.twofff[d.npass - 1];
     auto put = [&](auto add, int k, fx2 p, fx2 c) {   // c = P(M - k)
-        double2 a = fx_to(fx2{p.x + c.x, p.y - c.y}, ebp), b = fx_to(fx2{p.y + c.y, c.x - p.x}, ebp);
+        double2 a = fx_to(fx2{p.x + c.x, p.y - c.y}, n), b = fx_to(fx2{p.y + c.y, c.x - p.x}, n);
         if (scale != 1.0) {
             a = make_double2(a.x * scale, a.y * scale);
             b = make_double2(b.x * scale, b.y * scale);
         }
-        if constexpr (add.value) {   // (this thread alone reads and writes entry k)
-            double2 U = __ldcg(&urow[k]), V = __ldcg(&vrow[k]);
-            linear_part_bas(U, V, *reinterpret_cast<const double2*>(words + 4), 2.0 * M * scale, k == 0);
-            a = make_double2(a.x + U.x, a.y + U.y);
-            b = make_double2(b.x + V.x, b.y + V.y);
+        if constexpr (add.value) {
+            double2 U = make_double2(0.0, 0.0), V = U;
+            if (out) {   // (this thread alone reads and writes entry k)
+                U = __ldcg(&urow[k]);
+                V = __ldcg(&vrow[k]);
+                linear_part_bas(U, V, *means, 2.0 * M * scale, k == 0);
+            }
+            const double f = fx_rest(ebp);
+            a = make_double2(fma(a.x, f, U.x), fma(a.y, f, U.y));
+            b = make_double2(fma(b.x, f, V.x), fma(b.y, f, V.y));
         }
         urow[k] = a;
         vrow[k] = b;
@@ -336,14 +355,14 @@ __device__ __forceinline__ void fx_xpass_body(const Dims& d, double2* Iu, double
             }
         }
     };
-    if (out) split(std::true_type{});
+    if (out || n != ebp) split(std::true_type{});
     else split(std::false_type{});
 }
 
 // K3's transform: column kx of one product, read from the half-spectral rows
 // (mirrored radices, so that the retained rows are outputs 0 and 2 of the
-// last radix-3 butterflies).  sink(jc, value) gets the retained rows; SYNC: a
-// barrier between the last pass's loads and the sinks (which write to buf).
+// last radix-3 butterflies).  sink(jc) is where retained row jc goes, or null;
+// SYNC: a barrier between the last pass's loads and the stores (in buf).
 template <int E, bool SYNC, typename Sink>
 __device__ __forceinline__ void fx_yfwd_column(const Dims& d, const double2* __restrict__ I, bool active, int kx,
                                                const FxTw* __restrict__ tw, int g, int lane, longlong2* buf,
@@ -391,9 +410,12 @@ __device__ __forceinline__ void fx_yfwd_column(const Dims& d, const double2* __r
     int Ns = 4, t = 0;
     fx_middle<E, false>(buf, d, lane, T, tw, per, sum, kFxByLimit, Ns, t);
     const int tn = max(t, fx_shift_total(M, per, sum, kFxByLimit));
-    const int eb = fx_exponent_base(emax, 4, tn);
+    const int eb = fx_exponent_base(emax, 4, tn), n = fx_normal_base(eb);
     const FxTw* tp = tw + d.twofff[d.npass - 1];
     fx2 v[N3][3];
+    auto put = [&](int jc, fx2 z) {
+        if (double2* o = sink(jc)) *o = fx_to(z, n);
+    };
 #pragma unroll
     for (int b = 0; b < N3; ++b) {
         const int j = lane + b * T;
@@ -409,12 +431,24 @@ __device__ __forceinline__ void fx_yfwd_column(const Dims& d, const double2* __r
         fx_twiddle<3, false, true>(v[b], tp, K, j, tn - t);
         if (b == 0 && lane == 0) {
             fx_bf3<false>(v[b]);
-            sink(K, fx_to(v[b][1], eb));
+            put(K, v[b][1]);
         } else {
             fx_bf3_02<false>(v[b]);
         }
-        sink(j, fx_to(v[b][0], eb));
-        sink(j + K + 1, fx_to(v[b][2], eb));
+        put(j, v[b][0]);
+        put(j + K + 1, v[b][2]);
+    }
+    if (n != eb) {
+        const double f = fx_rest(eb);
+        auto again = [&](int jc) {
+            if (double2* o = sink(jc)) *o = make_double2(o->x * f, o->y * f);
+        };
+        if (lane == 0) again(K);
+#pragma unroll 1
+        for (int j = lane; j < K; j += T) {
+            again(j);
+            again(j + K + 1);
+        }
     }
 }
 
@@ -431,9 +465,8 @@ __device__ __forceinline__ void fx_yfwd_col_body(const Dims& d, const double2* _
     const bool active = kx < d.KX && g < G;
     double2* out = (f ? OutV : OutU) + (size_t)(active ? kx : 0) * d.ldS;
     fx_yfwd_column<E, false>(d, f ? Iv : Iu, active, kx, tw, g, lane,
-                             reinterpret_cast<longlong2*>(bufs + (size_t)g * d.M), [&](int jc, double2 v) {
-                                 if (active) out[jc] = v;
-                             });
+                             reinterpret_cast<longlong2*>(bufs + (size_t)g * d.M),
+                             [&](int jc) { return active ? out + jc : nullptr; });
 }
 
 // K3 in one kernel (see yfwd_body): 2G transforms, blockDim / T at a time,
@@ -452,7 +485,7 @@ __device__ __forceinline__ bool fx_yfwd_body(const Dims& d, const double2* __res
         const int i = t0 + t, f = i >= G, gg = i - f * G;   // buffer i: field f, column gg
         double2* buf = bufs + (size_t)i * d.M;
         fx_yfwd_column<E, true>(d, f ? Iv : Iu, gg < gtot, kx0 + gg, tw, t, lane, reinterpret_cast<longlong2*>(buf),
-                                [&](int jc, double2 v) { buf[jc] = v; });
+                                [&](int jc) { return buf + jc; });
         __syncthreads();
     }
     bool bad = false;

@@ -1,5 +1,5 @@
 """CPU test of the fixed-point results' conversion at both ends of FP64's range
-(fx_to_wide of csrc/s2d_fixed.cuh, which also compiles as C++): the same as
+(fx_to_normal and fx_rest of csrc/s2d_fixed.cuh, which also compiles as C++): the same as
 ldexp of the rounded integer, gradual underflow included."""
 
 import os
@@ -16,10 +16,10 @@ int main() {
     int bad = 0, low = 0;
     unsigned long long seed = 1;
     auto wide = [](long long x, int eb) {
-        const long long b = fx_to_wide(x, eb);
+        const long long b = fx_to_normal(x, fx_normal_base(eb));
         double v;
         memcpy(&v, &b, 8);
-        return v;
+        return fx_normal_base(eb) == eb ? v : v * fx_rest(eb);
     };
     for (int i = 0; i < 400000; ++i) {
         seed = seed * 6364136223846793005ULL + 1442695040888963407ULL;
